@@ -49,6 +49,7 @@
 #include "hs_channel.hpp"
 #include "hs_cht.hpp"
 #include "hs_mg.cuh"
+#include "hs_run.cuh"
 #include "hs_zm.cuh"
 
 namespace cg = cooperative_groups;
@@ -750,55 +751,55 @@ __device__ void mg_fine_and_rhs(const CgVec<M> &V, const mg::Level<M> &L0, doubl
   }
 }
 
-// The mixed form's two CG passes by runs of W consecutive padded cells of
-// an interior row per thread step (W = 2 or 4; aligned: the row pitch is a
-// multiple of four values), with 8- or 16-byte loads and stores: a fraction
-// 1/W of the load and store instructions of the per-cell passes, whose FP32
-// form was bound by them rather than by DRAM bytes.  Lanes outside the
-// interior (the ghost cells and the row's padding) compute from in-bounds
-// loads and store the zeros those cells hold.  Every interior cell's
-// arithmetic is the per-cell pass's, term for term; only the order of this
-// thread's dot-product terms differs.  Mixed p' solve per outer step at
-// 256x128x128: 3.39 ms per cell, 3.15 ms with W = 2, 3.11 ms with W = 4
-// (which spills 64 bytes at the kernel's 96 registers, and is still faster).
-constexpr int kCgRun = 4;
-
+// The CG's two passes by runs of W consecutive padded cells of an interior
+// row per thread step (16 bytes: two FP64 or four FP32 values; aligned: the
+// row pitch is a multiple of four values): a fraction of the load and store
+// instructions of per-cell passes, which bound them rather than DRAM.  Lanes
+// outside the interior (the ghost cells and the row's padding) compute from
+// in-bounds loads and store the zeros those cells hold.  Every interior
+// cell's arithmetic is the per-cell pass's, term for term; only the order of
+// this thread's dot-product terms differs.  Per cell the mixed p' solve took
+// 3.39 ms per outer step at 256x128x128 against 3.11 by runs.
 template <int W>
 __device__ __forceinline__ void ldv(float (&v)[W], const float *p, bool cg_) {
-  if constexpr (W == 4) {
-    const float4 t = cg_ ? __ldcg(reinterpret_cast<const float4 *>(p)) : *reinterpret_cast<const float4 *>(p);
-    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-  } else {
-    const float2 t = cg_ ? __ldcg(reinterpret_cast<const float2 *>(p)) : *reinterpret_cast<const float2 *>(p);
-    v[0] = t.x; v[1] = t.y;
-  }
+  const float4 t = cg_ ? __ldcg(reinterpret_cast<const float4 *>(p)) : *reinterpret_cast<const float4 *>(p);
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+template <int W>
+__device__ __forceinline__ void ldv(double (&v)[W], const double *p, bool cg_) {
+  const double2 t = cg_ ? __ldcg(reinterpret_cast<const double2 *>(p)) : *reinterpret_cast<const double2 *>(p);
+  v[0] = t.x; v[1] = t.y;
 }
 template <int W>
 __device__ __forceinline__ void stv(float *p, const float (&v)[W]) {
-  if constexpr (W == 4) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-  else *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+template <int W>
+__device__ __forceinline__ void stv(double *p, const double (&v)[W]) {
+  *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
 }
 // p = z + beta p_old (or z in the first iteration) at the run q0
-template <int W>
-__device__ __forceinline__ void p_run(float (&v)[W], const float *zs, const float *po, int q0, bool first, float bm) {
-  ldv<W>(v, zs + q0, true);
+template <class M, int W>
+__device__ __forceinline__ void p_run(M (&v)[W], const M *zs, const M *po, int q0, bool first, M bm) {
+  ldv(v, zs + q0, false);
   if (!first) {
-    float o[W];
-    ldv<W>(o, po + q0, true);
+    M o[W];
+    ldv(o, po + q0, false);
 #pragma unroll
     for (int c = 0; c < W; ++c) v[c] = v[c] + bm * o[c];
   }
 }
-__device__ __forceinline__ float p_one(const float *zs, const float *po, int q, bool first, float bm) {
-  const float z = __ldcg(zs + q);
-  return first ? z : z + bm * __ldcg(po + q);
+template <class M>
+__device__ __forceinline__ M p_one(const M *zs, const M *po, int q, bool first, M bm) {
+  const M z = zs[q];
+  return first ? z : z + bm * po[q];
 }
 
 // s = A p with the new p formed on the way (k_ch_pcg's first pass); returns
 // this thread's share of <s, p>
-template <int W>
-__device__ double cg_ap_runs(const CgVec<float> &V, const float *zs, const float *po, float *pn, bool first, float bm,
-                             int tid, int T) {
+template <class M>
+__device__ double cg_ap_runs(const CgVec<M> &V, const M *zs, const M *po, M *pn, bool first, M bm, int tid, int T) {
+  constexpr int W = run::Run<M>::W;
   const int N0 = V.N0, PX = V.px, PY = V.N1 + 2, PXY = V.px * (V.N1 + 2);
   double acc = 0.0;
   for (mg::Walk w(PX / W, V.N1, V.N2, tid, T); w.ok(); w.next()) {
@@ -806,14 +807,14 @@ __device__ double cg_ap_runs(const CgVec<float> &V, const float *zs, const float
     // the sums d = cw + ce + cs + cn + cb + cf and o = cw pW + ce pE + cs pS
     // + cn pN + cb pB + cf pF built up in that order, one neighbour run at a
     // time (fewer values live at once)
-    float pc[W + 2], g[W + 1], v[W], h[W];
+    M pc[W + 2], g[W + 1], v[W], h[W];
     double d[W], o[W];
-    p_run<W>(v, zs, po, q0, first, bm);
+    p_run(v, zs, po, q0, first, bm);
     pc[0] = p_one(zs, po, q0 - 1, first, bm);
 #pragma unroll
     for (int c = 0; c < W; ++c) pc[c + 1] = v[c];
     pc[W + 1] = p_one(zs, po, q0 + W, first, bm);
-    ldv<W>(v, V.acx + q0, false);
+    ldv(v, V.acx + q0, false);
 #pragma unroll
     for (int c = 0; c < W; ++c) g[c] = v[c];
     g[W] = V.acx[q0 + W];
@@ -822,35 +823,35 @@ __device__ double cg_ap_runs(const CgVec<float> &V, const float *zs, const float
       d[c] = (double)g[c] + (double)g[c + 1];
       o[c] = (double)g[c] * (double)pc[c] + (double)g[c + 1] * (double)pc[c + 2];
     }
-    p_run<W>(v, zs, po, q0 - PX, first, bm);
-    ldv<W>(h, V.acy + q0, false);
+    p_run(v, zs, po, q0 - PX, first, bm);
+    ldv(h, V.acy + q0, false);
 #pragma unroll
     for (int c = 0; c < W; ++c) { d[c] = d[c] + (double)h[c]; o[c] = o[c] + (double)h[c] * (double)v[c]; }
-    p_run<W>(v, zs, po, q0 + PX, first, bm);
-    ldv<W>(h, V.acy + q0 + PX, false);
+    p_run(v, zs, po, q0 + PX, first, bm);
+    ldv(h, V.acy + q0 + PX, false);
 #pragma unroll
     for (int c = 0; c < W; ++c) { d[c] = d[c] + (double)h[c]; o[c] = o[c] + (double)h[c] * (double)v[c]; }
-    p_run<W>(v, zs, po, q0 - PXY, first, bm);
-    ldv<W>(h, V.acz + q0, false);
+    p_run(v, zs, po, q0 - PXY, first, bm);
+    ldv(h, V.acz + q0, false);
 #pragma unroll
     for (int c = 0; c < W; ++c) { d[c] = d[c] + (double)h[c]; o[c] = o[c] + (double)h[c] * (double)v[c]; }
-    p_run<W>(v, zs, po, q0 + PXY, first, bm);
-    ldv<W>(h, V.acz + q0 + PXY, false);
-    float pv[W], sv[W];
+    p_run(v, zs, po, q0 + PXY, first, bm);
+    ldv(h, V.acz + q0 + PXY, false);
+    M pv[W], sv[W];
 #pragma unroll
     for (int c = 0; c < W; ++c) {
       d[c] = d[c] + (double)h[c];
       o[c] = o[c] + (double)h[c] * (double)v[c];
       const int i = W * w.m + c;  // padded x
       const bool in = i >= 1 && i <= N0;
-      const float p0 = pc[c + 1];
+      const M p0 = pc[c + 1];
       const double s_ = d[c] * (double)p0 - o[c];
-      pv[c] = in ? p0 : 0.0f;
-      sv[c] = in ? (float)s_ : 0.0f;
-      if (in) acc += (double)(float)s_ * (double)p0;
+      pv[c] = in ? p0 : M(0);
+      sv[c] = in ? (M)s_ : M(0);
+      if (in) acc += (double)(M)s_ * (double)p0;
     }
-    stv<W>(pn + q0, pv);
-    stv<W>(V.s + q0, sv);
+    stv(pn + q0, pv);
+    stv(V.s + q0, sv);
   }
   return acc;
 }
@@ -859,42 +860,39 @@ __device__ double cg_ap_runs(const CgVec<float> &V, const float *zs, const float
 // side r and the seed of the first half-sweep (x = r / d on colour 0; colour
 // 1, which the next half-sweep writes before any pass reads it, gets 0);
 // returns this thread's share of <r, r>
-template <int W>
-__device__ double cg_update_runs(const CgVec<float> &V, const mg::Level<float> &L0, bool pre, const float *pn,
-                                 double alpha, int tid, int T) {
+template <class M>
+__device__ double cg_update_runs(const CgVec<M> &V, const mg::Level<M> &L0, bool pre, const M *pn, double alpha,
+                                 int tid, int T) {
+  constexpr int W = run::Run<M>::W;
   const int N0 = V.N0, PX = V.px, PY = V.N1 + 2;
   double acc = 0.0;
   for (mg::Walk w(PX / W, V.N1, V.N2, tid, T); w.ok(); w.next()) {
     const int q0 = W * w.m + PX * ((w.j + 1) + PY * (w.k + 1));
-    float xv[W], pv[W], rv[W], sv[W], dv[W];
-    ldv<W>(xv, V.x + q0, false);
-    ldv<W>(pv, pn + q0, false);
-    ldv<W>(rv, V.r + q0, false);
-    ldv<W>(sv, V.s + q0, false);
-    if (pre) ldv<W>(dv, L0.d + q0, false);
+    M xv[W], pv[W], rv[W], sv[W], dv[W];
+    ldv(xv, V.x + q0, false);
+    ldv(pv, pn + q0, false);
+    ldv(rv, V.r + q0, false);
+    ldv(sv, V.s + q0, false);
+    if (pre) ldv(dv, L0.d + q0, false);
     else
 #pragma unroll
-      for (int c = 0; c < W; ++c) dv[c] = 0.0f;
-    float xo[W], ro[W], sx[W];
+      for (int c = 0; c < W; ++c) dv[c] = M(0);
+    M xo[W], ro[W], sx[W];
 #pragma unroll
     for (int c = 0; c < W; ++c) {
       const int i = W * w.m + c;
       const bool in = i >= 1 && i <= N0;
-      const float xn = (float)((double)xv[c] + alpha * (double)pv[c]);
-      const float rn = (float)((double)rv[c] - alpha * (double)sv[c]);
+      const M xn = (M)((double)xv[c] + alpha * (double)pv[c]);
+      const M rn = (M)((double)rv[c] - alpha * (double)sv[c]);
       xo[c] = in ? xn : xv[c];
       ro[c] = in ? rn : rv[c];
       if (in) acc += (double)rn * (double)rn;
       const bool red = in && !(((i - 1) + w.j + w.k) & 1);
-      sx[c] = red ? (dv[c] == 0.0f ? 0.0f : rn / dv[c]) : 0.0f;
-      rv[c] = in ? rn : 0.0f;
+      sx[c] = red ? (dv[c] == M(0) ? M(0) : rn / dv[c]) : M(0);
     }
-    stv<W>(V.x + q0, xo);
-    stv<W>(V.r + q0, ro);
-    if (pre) {
-      stv<W>(L0.rhs + q0, rv);
-      stv<W>(L0.x + q0, sx);
-    }
+    stv(V.x + q0, xo);
+    stv(V.r + q0, ro);
+    if (pre) stv(L0.x + q0, sx);
   }
   return acc;
 }
@@ -905,8 +903,9 @@ __device__ double cg_update_runs(const CgVec<float> &V, const mg::Level<float> &
 // forms the new p of its cell and of the six neighbours from z and the old
 // p; p is double-buffered), and <r, z> inside the V-cycle's last pass.
 template <class M>
-__global__ void __launch_bounds__(PcgT<M>::v, 1) k_ch_pcg(CgVec<M> V, mg::Hier<M> G, int precond, double tol, int maxiter, double *partials,
-                                               int *out_it, double *out_rel) {
+__global__ void __launch_bounds__(PcgT<M>::v, 1)
+    k_ch_pcg(const __grid_constant__ CgVec<M> V, const __grid_constant__ mg::Hier<M> G, int precond, double tol,
+             int maxiter, double *partials, int *out_it, double *out_rel) {
   cg::grid_group grid = cg::this_grid();
   __shared__ double sh[40];
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
@@ -929,15 +928,25 @@ __global__ void __launch_bounds__(PcgT<M>::v, 1) k_ch_pcg(CgVec<M> V, mg::Hier<M
   }
   if (precond) mg::build(G, false, grid, tid, T);
   const double eps = tol * tol;
-  // gamma = <r, z>
-  auto rz = [&]() {
+  // gamma = <r, z>, summed in the V-cycle's last per-cell pass, or, after run
+  // passes, in a pass of its own in that pass's order
+  auto rz = [&]() __attribute__((always_inline)) {
     double a = 0.0;
     if (!precond) return bb;
-    if (!mg::vcycle<M, M, true>(G, false, grid, tid, T, V.r, &a))
+    if (is_mixed(M()) && G.nrun > 0) {
+      if constexpr (is_mixed(M())) run::vcycle<true>(G, grid, tid, T);
+      for (mg::Walk w((N0 + 1) / 2, N1, V.N2, tid, T); w.ok(); w.next()) {
+        const int h = (w.j + w.k) & 1, i = 2 * w.m + h, ib = 2 * w.m + (h ^ 1);
+        const int q0 = 2 * w.m + 1 + PX * ((w.j + 1) + PY * (w.k + 1));
+        if (i < N0) a += (double)V.r[q0 + h] * (double)L0.x[q0 + h];
+        if (ib < N0) a += (double)V.r[q0 + (h ^ 1)] * (double)L0.x[q0 + (h ^ 1)];
+      }
+    } else if (!mg::vcycle<M, M, true>(G, false, grid, tid, T, V.r, &a)) {
       for (mg::Walk w(N0, N1, V.N2, tid, T); w.ok(); w.next()) {
         const int q = (w.m + 1) + PX * ((w.j + 1) + PY * (w.k + 1));
         a += (double)V.r[q] * (double)__ldcg(L0.x + q);
       }
+    }
     return grid_sum(a, partials, buf, sh, grid);
   };
   double gamma = rz(), rr = bb, beta = 0.0;
@@ -946,41 +955,14 @@ __global__ void __launch_bounds__(PcgT<M>::v, 1) k_ch_pcg(CgVec<M> V, mg::Hier<M
   while (it < maxiter && !(rr / bb < eps)) {
     const bool first = it == 0;
     it++;
-    acc = 0.0;
     const M bm = (M)beta;
-    auto pval = [&](int qq) -> M {
-      const M z = precond ? __ldcg(L0.x + qq) : __ldcg(V.r + qq);
-      return first ? z : z + bm * __ldcg(po + qq);
-    };
     // p in storage precision; the product in FP64 (in FP32 its cancellation
     // error for smooth p would reach the near-null modes of the p' system)
-    if constexpr (is_mixed(M())) acc = cg_ap_runs<kCgRun>(V, precond ? L0.x : V.r, po, pn, first, bm, tid, T);
-    else for (mg::Walk w(N0, N1, V.N2, tid, T); w.ok(); w.next()) {
-      const int q = (w.m + 1) + PX * ((w.j + 1) + PY * (w.k + 1));
-      const M p0 = pval(q);
-      const double cw = V.acx[q], ce = V.acx[q + 1], cs = V.acy[q], cn = V.acy[q + PX], cb = V.acz[q], cf = V.acz[q + PXY];
-      const double d = cw + ce + cs + cn + cb + cf;
-      const double sv = d * (double)p0 - (cw * (double)pval(q - 1) + ce * (double)pval(q + 1) + cs * (double)pval(q - PX) +
-                                          cn * (double)pval(q + PX) + cb * (double)pval(q - PXY) + cf * (double)pval(q + PXY));
-      pn[q] = p0;
-      V.s[q] = (M)sv;
-      acc += (double)(M)sv * (double)p0;
-    }
+    acc = cg_ap_runs(V, (const M *)(precond ? L0.x : V.r), (const M *)po, pn, first, bm, tid, T);
     const double sp = grid_sum(acc, partials, buf, sh, grid);
     if (sp == 0.0) break;
     const double alpha = gamma / sp;
-    acc = 0.0;
-    if constexpr (is_mixed(M())) acc = cg_update_runs<kCgRun>(V, L0, precond != 0, pn, alpha, tid, T);
-    else for (mg::Walk w(N0, N1, V.N2, tid, T); w.ok(); w.next()) {
-      const int q = (w.m + 1) + PX * ((w.j + 1) + PY * (w.k + 1));
-      const double xv = (double)V.x[q], pv = (double)pn[q], r0 = (double)V.r[q], sv = (double)V.s[q];
-      const mg::Seed<M> sd = precond ? mg::seed_at(L0, w.m, w.j, w.k, q, false) : mg::Seed<M>{};
-      V.x[q] = (M)(xv + alpha * pv);
-      const M rv = (M)(r0 - alpha * sv);
-      V.r[q] = rv;
-      acc += (double)rv * (double)rv;
-      if (precond) sd.store(L0, q, rv);
-    }
+    acc = cg_update_runs(V, L0, precond != 0, (const M *)pn, alpha, tid, T);
     rr = grid_sum(acc, partials, buf, sh, grid);
     if (rr / bb < eps || it >= maxiter) break;  // no V-cycle for an iteration that will not run
     const double gnew = precond ? rz() : rr;
@@ -1396,15 +1378,23 @@ void setup_cg(ChannelState &S, CgVec<R> &V, const uint8_t *solid, size_t np) {
   V.r2 = S.alloc<R>(np);
 }
 
+// The smallest level in run passes (hs_run.cuh).  A smaller one's pass is a
+// grid barrier and a round trip of loads, which the per-cell passes spread
+// over more threads: 128x64x64 alone takes 3.9 us per half-sweep per cell and
+// 4.0-4.2 by runs; 203x75x110 (1.7 million cells) gains (hs_run.cuh).
+constexpr long long kRunCells = 1000000;
+
 template <class M>
-void setup_mg(ChannelState &S, mg::Hier<M> &G, const CgVec<M> &V) {
+void setup_mg(ChannelState &S, mg::Hier<M> &G, const CgVec<M> &V, int nsm) {
   int nx = S.N0, ny = S.N1, nz = S.N2, L = 0;
   while (true) {
     if (L >= mg::kMgMaxLv) throw std::runtime_error("multigrid: too many levels");
     mg::Level<M> &l = G.lv[L];
     l.nx = nx; l.ny = ny; l.nz = nz; l.px = pitch4(nx + 2);
     const size_t np = (size_t)l.px * (ny + 2) * (nz + 2);
-    l.x = S.alloc<M>(np); l.rhs = S.alloc<M>(np);
+    l.x = S.alloc<M>(np);
+    // level 0's rhs is the CG's residual (the z-marching form keeps a buffer of its own there)
+    l.rhs = L == 0 && S.prm.p_level0 != 2 ? V.r : S.alloc<M>(np);
     if (L == 0) {  // the p' couplings themselves (written by the assembly, read-only in the solve)
       l.gx = const_cast<M *>(V.acx); l.gy = const_cast<M *>(V.acy); l.gz = const_cast<M *>(V.acz);
       l.d = S.alloc<M>(np);
@@ -1427,6 +1417,14 @@ void setup_mg(ChannelState &S, mg::Hier<M> &G, const CgVec<M> &V) {
   G.nswc = G.nsw + 1;
   G.lu = S.alloc<double>((size_t)mg::kMgCoarse * mg::kMgCoarse);
   mg::plan_stage(G);
+  // mixed form: run passes on the levels of at least kRunCells cells
+  G.nrun = 0;
+  if constexpr (is_mixed(M()))
+    while (S.prm.p_level0 == 0 && G.nrun < G.ls &&
+           (long long)G.lv[G.nrun].nx * G.lv[G.nrun].ny * G.lv[G.nrun].nz >= kRunCells) {
+      G.zc[G.nrun] = run::pick_planes(G.lv[G.nrun], nsm * PcgT<M>::v / 32);
+      ++G.nrun;
+    }
 }
 
 // ---- TMA tensor maps (the driver's encoder, reached through the runtime)
@@ -1648,10 +1646,10 @@ ChannelState *ch_create(const Case &c, const ChParams &p, int device) {
   if (S->mixed) setup_cg(*S, S->Vf, solid, np);
   else setup_cg(*S, S->Vd, solid, np);
   S->scratch = S->alloc<double>(np);
-  if (S->mixed) setup_mg(*S, S->Gf, S->Vf);
-  else setup_mg(*S, S->Gd, S->Vd);
   int per = 0, nsm = 0;
   CH_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+  if (S->mixed) setup_mg(*S, S->Gf, S->Vf, nsm);
+  else setup_mg(*S, S->Gd, S->Vd, nsm);
   // momentum: a grid resident at once (its three components of a chunk of
   // faces in consecutive blocks then march through the z-planes together:
   // 0.71 -> 0.66 ms per FP64 momentum solve at 256x128x128 against 3 x 1184

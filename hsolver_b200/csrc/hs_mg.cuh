@@ -64,6 +64,8 @@ struct Hier {
   int ls;      // first level that block 0 handles alone (plan_stage)
   int stage;   // bytes of dynamic shared memory holding x and rhs of levels ls..L-1 and the read-only arrays
   int sx[kMgMaxLv], sr[kMgMaxLv];  // byte offsets of a staged level's x and rhs in it
+  int nrun;        // levels 0..nrun - 1 are smoothed by runs (hs_run.cuh; the p' solve's large levels)
+  int zc[kMgMaxLv];  // their planes per unit
   int sro;     // first level whose couplings, fluxes and mask are staged too (L: none)
   int sg[kMgMaxLv][3], sf[kMgMaxLv][3], sm[kMgMaxLv];  // their byte offsets (-1: the array is null)
 };
