@@ -4,13 +4,13 @@
 // lexicographic order (k outer, j, i inner; fluid_solver.h:419-421,
 // 505-507, 588-590, 807-809; mobs_solver.h:477-479).  With a 7-point
 // dependency, cell (i,j,k) reads new values at (i-1,j,k), (i,j-1,k),
-// (i,j,k-1) and old values at (i+1,j,k), (i,j+1,k), (i,j,k+1).  Cells on
-// the hyperplane i+j+k = s therefore depend only on hyperplane s-1, so the
-// sweep runs as a wavefront: one cooperative kernel per solve, one grid-wide
-// barrier per hyperplane, one thread per (j,k) row.  Every point update uses
-// the reference's arithmetic in the reference's operation order (the build
-// disables FMA contraction), so the sweep is the reference's sweep, not an
-// approximation of it.
+// (i,j,k-1) and old values at (i+1,j,k), (i,j+1,k), (i,j,k+1).  So the rows
+// (j,k) are cut into tiles of one warp each that march along i one step
+// behind their j - 1 and k - 1 neighbours (a wavefront), the tiles waiting on
+// one another's progress counters instead of on grid barriers.  Every point
+// update uses the reference's arithmetic in the reference's operation order
+// (the build disables FMA contraction), so the sweep is the reference's sweep,
+// not an approximation of it.
 //
 // Pressure correction.  Matrix-free CG over the fluid cells with HYPRE
 // PCG's recurrences and stopping rule (identity preconditioner, two-norm,
@@ -91,6 +91,9 @@ struct DevStats {
   double pcg_relres;
   int solid_sweeps_max;
   int pad;
+  // the solve that k_gs_tiles leaves to k_gs_planes: its sweeps and residuals so far
+  int gs_open, gs_done;
+  double gs_residual, gs_res;
   // running totals since creation (bench byte accounting)
   long long cum_sweeps[4];
   long long cum_solid_cell_sweeps;
@@ -309,16 +312,27 @@ __device__ __forceinline__ double upd_w(const FluidDev &F, const Prm &P, int i, 
   return P.relax * nv + (1 - P.relax) * old;
 }
 
-// ---------------------------------------------------------------- pipelined exact Gauss-Seidel
-// Consecutive lexicographic sweeps overlap: sweep n+1 may update hyperplane
-// s once sweep n has finished hyperplane s+1 (it needs sweep n's values at
-// i+1, j+1, k+1 and its own new values at i-1, j-1, k-1).  At time t sweep
-// n therefore works on hyperplane t - 2n; every read is of a value written at
-// an earlier time step, so one grid barrier per time step suffices and W
-// sweeps take S + 2(W-1) steps instead of W*S.
+// ---------------------------------------------------------------- wavefront Gauss-Seidel
+// A tile is 8 x 4 rows (j, k); lane (jj, kk) of its warp updates i = s - jj -
+// kk + 1 at step s, so the new values at j - 1 and k - 1 inside the tile are
+// the neighbouring lanes' results of the step before (shuffles) and the one at
+// i - 1 is its own.  The tile's lower edges come from the tiles (J-1, K) and
+// (J, K-1) through memory.  Progress is counted in chunks of kGsCh steps: a
+// warp starts a chunk once those tiles have passed the steps it reads, which
+// is about two chunks behind each; a release store per chunk publishes its
+// own.  The old values and the other fields are staged in shared memory a
+// chunk ahead, eight consecutive i of a row per eight lanes: a lane's own
+// loads would touch 32 lines per instruction (1.3 ms per momentum sweep at
+// 256x128x128).
 //
-// The reference decides after each sweep whether to sweep again (residual
-// test, fluid_solver.h:414-416).  A window of W sweeps is therefore
+// A grid barrier per hyperplane i+j+k costs ~5 us with its dependent loads
+// (510 of them at 256x128x128: 2.85 ms per momentum sweep); here a step costs
+// one update's latency and a hop between tiles a flag's.
+//
+// Several sweeps overlap: sweep n of a tile starts a chunk once the tiles
+// (J+1, K) and (J, K+1) have finished it in sweep n - 1 (their old values
+// here).  The reference decides after each sweep whether to sweep again
+// (residual test, fluid_solver.h:414-416).  A window of W sweeps is therefore
 // speculative: the per-sweep residual sums are kept separately, the stop
 // test is replayed sweep by sweep, and if the reference would have stopped
 // inside the window the field is restored from a snapshot and exactly that
@@ -329,6 +343,426 @@ __device__ __forceinline__ double upd_w(const FluidDev &F, const Prm &P, int i, 
 // 656) only rewrite values the sweeps never change, except that applyY sets
 // the lid row of u to U0 after the first v sweep; later v sweeps read U0
 // there directly (`lid`), and each BC is applied once after the solve.
+constexpr int kTJ = 8, kTK = 4;  // rows of a tile
+constexpr int kGsCh = 8;         // steps per chunk
+constexpr int kGsT = 128;        // threads per block: four warps, spread over the SMs first
+// The window size up to which a solve runs by tiles: a tile's chunk costs its
+// flag, edge loads and release store (~4 us) on top of its steps whatever the
+// number of sweeps, the hyperplane form's barrier serves every sweep in
+// flight (256x128x128 energy: one sweep 0.5 against 1.6 ms, 100 sweeps 34
+// against 15).
+constexpr int kTileW = 4;
+constexpr int kGsSpin = 1 << 21; // polls before a wait gives up (about a second)
+constexpr int kGsRing = 32, kGsPitch = 35;  // i values per staged row; its pitch (the lanes' rows and skew in distinct banks)
+
+// The staged arrays of an equation: its own field and the three others it
+// reads (u, v, w and p without its own; the energy u, v, w), each as nj x nk
+// rows from (j + dj, k + dk) on
+struct GsRows {
+  int nj, nk, dj, dk;
+  __host__ __device__ constexpr int n() const { return nj * nk; }
+};
+template <int EQ>
+__host__ __device__ constexpr GsRows gs_rows(int a) {
+  if (a == 0) return {kTJ + 1, kTK + 1, 0, 0};
+  if (EQ == 0) return a == 1 ? GsRows{kTJ + 1, kTK, 0, 0} : a == 2 ? GsRows{kTJ, kTK + 1, 0, 0} : GsRows{kTJ, kTK, 0, 0};
+  if (EQ == 1) return a == 2 ? GsRows{kTJ + 1, kTK + 1, -1, 0} : GsRows{kTJ + 1, kTK, -1, 0};
+  if (EQ == 2) return a == 2 ? GsRows{kTJ + 1, kTK + 1, 0, -1} : GsRows{kTJ, kTK + 1, 0, -1};
+  return {kTJ, kTK, 0, 0};
+}
+template <int EQ>
+__host__ __device__ constexpr int gs_base(int a) {  // first staged row of array a; a = 4: their number
+  int n = 0;
+  for (int q = 0; q < a; ++q) n += gs_rows<EQ>(q).n();
+  return n;
+}
+constexpr int kGsGeo = 5;  // staged rows of x geometry
+// geometry array a along x: widths and the reciprocals of the distances
+template <int EQ>
+__device__ __forceinline__ const double *gs_geo(const FluidDev &F, int a) {
+  if (EQ == 3) return a == 0 ? F.xp : a == 1 ? F.xw : a == 2 ? F.rsx : F.ix2;
+  return a == 0 ? F.xp : a == 1 ? F.xw : a == 2 ? F.xe : a == 3 ? F.rxw : F.rxe;
+}
+// shared memory of a block: the staged rows of its warps
+template <int EQ>
+constexpr int gs_smem() { return (gs_base<EQ>(4) + kGsGeo) * kGsPitch * 8 * (kGsT / 32); }
+
+template <int EQ>
+__device__ __forceinline__ int gs_idx(const FluidDev &F, int i, int j, int k) {
+  return EQ == 0 ? IU(F, i, j, k) : EQ == 1 ? IV(F, i, j, k) : EQ == 2 ? IW(F, i, j, k) : IP(F, i, j, k);
+}
+// array a of equation EQ at (i, j, k)
+template <int EQ, int A>
+__device__ __forceinline__ const double *gs_at(const FluidDev &F, int i, int j, int k) {
+  constexpr int f = A == 0 ? EQ : EQ == 3 ? A - 1 : A == 3 ? 3 : A - 1 + (A - 1 >= EQ);  // 0 u, 1 v, 2 w, 3 p (the energy's own: T)
+  if constexpr (A == 0) return (EQ == 0 ? F.u : EQ == 1 ? F.v : EQ == 2 ? F.w : F.tt) + gs_idx<EQ>(F, i, j, k);
+  else if constexpr (f == 0) return F.u + IU(F, i, j, k);
+  else if constexpr (f == 1) return F.v + IV(F, i, j, k);
+  else if constexpr (f == 2) return F.w + IW(F, i, j, k);
+  else return F.pt + IP(F, i, j, k);
+}
+
+// the values of one update: the old ones of the own field at i (c), i + 1, j + 1,
+// k + 1, the other fields at i (x) and at i - 1 (cx)
+template <int EQ>
+struct GsIn {
+  static constexpr int NX = EQ == 0 ? 5 : EQ == 3 ? 3 : 8;
+  double c, e, n, b, x[NX], cx[NX];
+  double g[kGsGeo];  // gs_geo at i
+};
+
+// The update of cell (i, j, k) from the new values w, s, m at i - 1, j - 1,
+// k - 1 and `in`.  Bodies of solveXmomentum
+// (fluid_solver.h:591-624), solveYmomentum (508-541), solveZmomentum (422-455)
+// and solveTemp (810-846).
+template <int EQ>
+__device__ __forceinline__ double gs_update(const FluidDev &F, const Prm &P, int i, int j, int k, double w, double s,
+                                            double m, const GsIn<EQ> &in, bool lid, double &ap) {
+  const double c = in.c;
+  const double *cx = in.cx;
+  const double xp = in.g[0], xw = in.g[1];
+  const double yp = __ldg(F.yp + j), ys = __ldg(F.ys + j), zp = __ldg(F.zp + k), zf = __ldg(F.zf + k);
+  if constexpr (EQ == 3) {
+    const double sx = (xp + xw) / 2.0, sy = (yp + ys) / 2.0, sz = (zp + zf) / 2.0;
+    const double conv = -in.x[0] * (in.e - w) - in.x[1] * (in.n - s) - in.x[2] * (in.b - m);
+    const double rx = in.g[2], ry = __ldg(F.rsy + j), rz = __ldg(F.rsz + k);
+    // alpha*(te+tw)/sx/sx etc. (fluid_solver.h:838-840) with exact divisions
+    const double diff = div_pre(div_pre(P.alpha * (in.e + w), sx, rx), sx, rx) +
+                        div_pre(div_pre(P.alpha * (in.n + s), sy, ry), sy, ry) +
+                        div_pre(div_pre(P.alpha * (in.b + m), sz, rz), sz, rz);
+    const double denom = 2 * P.alpha * (in.g[3] + __ldg(F.iy2 + j) + __ldg(F.iz2 + k));
+    return (conv + diff) / denom * (P.relax) + (1 - P.relax) * c;
+  } else {
+    const double xe = in.g[2], yn = __ldg(F.yn + j), zb = __ldg(F.zb + k);
+    const double facexy = xp * yp, facexz = xp * zp, faceyz = yp * zp;
+    const double Dw = div_pre(2 * P.nu * faceyz, xp + xw, in.g[3]), De = div_pre(2 * P.nu * faceyz, xp + xe, in.g[4]);
+    const double Ds = div_pre(2 * P.nu * facexz, ys + yp, __ldg(F.rys + j)), Dn = div_pre(2 * P.nu * facexz, yn + yp, __ldg(F.ryn + j));
+    const double Db = div_pre(2 * P.nu * facexy, zb + zp, __ldg(F.rzb + k)), Df = div_pre(2 * P.nu * facexy, zf + zp, __ldg(F.rzf + k));
+    double fw, fe, fs, fn, fb, ff, b;
+    if constexpr (EQ == 0) {
+      fw = 0.5 * P.rho * faceyz * (c + w);
+      fe = 0.5 * P.rho * faceyz * (c + in.e);
+      fs = 0.5 * P.rho * facexz * (in.x[0] + cx[0]);
+      fn = 0.5 * P.rho * facexz * (in.x[1] + cx[1]);
+      fb = 0.5 * P.rho * facexy * (in.x[3] + cx[3]);
+      ff = 0.5 * P.rho * facexy * (in.x[2] + cx[2]);
+      b = faceyz * (cx[4] - in.x[4]);
+    } else if constexpr (EQ == 1) {
+      // the lid row of u (j == cy, 1 <= i <= cx) reads U0 once applyY has run (after v sweep 1)
+      const bool at_lid = lid && j == F.cy;
+      const double u_c = at_lid ? P.u_lid : cx[0];
+      const double u_e = (at_lid && i + 1 <= F.cx) ? P.u_lid : in.x[0];
+      fn = 0.5 * P.rho * facexz * (c + s);
+      fs = 0.5 * P.rho * facexz * (c + in.n);
+      fe = 0.5 * P.rho * faceyz * (u_c + cx[1]);
+      fw = 0.5 * P.rho * faceyz * (u_e + in.x[1]);
+      fb = 0.5 * P.rho * facexy * (in.x[2] + in.x[3]);
+      ff = 0.5 * P.rho * facexy * (in.x[4] + in.x[5]);
+      b = facexz * (in.x[6] - in.x[7]);
+    } else {
+      fb = 0.5 * P.rho * facexy * (c + m);
+      ff = 0.5 * P.rho * facexy * (c + in.b);
+      fw = 0.5 * P.rho * faceyz * (cx[0] + cx[1]);
+      fe = 0.5 * P.rho * faceyz * (in.x[0] + in.x[1]);
+      fs = 0.5 * P.rho * facexz * (in.x[2] + in.x[3]);
+      fn = 0.5 * P.rho * facexz * (in.x[4] + in.x[5]);
+      b = facexy * (in.x[6] - in.x[7]);
+    }
+    const double ae = De + dmax0(-fe), aw = Dw + dmax0(fw), an = Dn + dmax0(-fn);
+    const double as = Ds + dmax0(fs), ab = Db + dmax0(-fb), af = Df + dmax0(ff);
+    ap = ae + aw + an + as + ab + af;
+    const double nv = (ae * in.e + aw * w + an * in.n + as * s + af * m + ab * in.b + b) / ap;
+    return P.relax * nv + (1 - P.relax) * c;
+  }
+}
+
+// A warp's view of the tiles' progress (chunks finished, counted over the sweeps of the window)
+struct GsFlags {
+  int *prog;       // one per tile
+  int *give_up;    // set by the first wait that runs out; no wait is taken after it
+  bool dead;
+  // lanes 0..3 hold one tile index and the count it must have reached (idx < 0: none)
+  __device__ __forceinline__ void wait(int idx, int need) {
+    if (!dead) {
+      int spins = 0;
+      while (true) {
+        int v = need;
+        if (idx >= 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(prog + idx) : "memory");
+        if (__all_sync(0xffffffffu, v >= need)) break;
+        ++spins;
+        if ((spins & 1023) == 0 && (spins >= kGsSpin || *(volatile int *)give_up)) {
+          dead = true;
+          break;
+        }
+      }
+      if (dead && (threadIdx.x & 31) == 0) *(volatile int *)give_up = 1;
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ void done(int tile, int count) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+      asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(prog + tile), "r"(count) : "memory");
+  }
+};
+
+// Stages array A's rows of the tile at (j0, k0) for chunk ch: of the row at
+// lane position (rj, rk) the values i = kGsCh ch + 2 - rj - rk ... + kGsCh - 1,
+// eight lanes a row.  The own field, which other SMs write, through L2 into
+// registers (t), the others by asynchronous copies.
+template <int EQ, int A>
+__device__ __forceinline__ void gs_stage(const FluidDev &F, double *sm, int ch, int j0, int k0, int NI, int NJ, int NK,
+                                         double *t) {
+  constexpr GsRows R = gs_rows<EQ>(A);
+  double *ring = sm + gs_base<EQ>(A) * kGsPitch;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < (R.n() + 3) / 4; ++q) {
+    const int r = 4 * q + lane / 8, rj = r % R.nj, rk = r / R.nj;
+    const int i = kGsCh * ch + 2 - (rj + R.dj) - (rk + R.dk) + lane % 8, j = j0 + rj + R.dj, k = k0 + rk + R.dk;
+    const bool ok = r < R.n() && i >= 0 && i <= NI + 1 && j <= NJ + 1 && k <= NK + 1;
+    if constexpr (A == 0) {
+      t[q] = ok ? ld(gs_at<EQ, A>(F, i, j, k)) : 0.0;
+    } else if (ok) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(ring + r * kGsPitch + (i & (kGsRing - 1)));
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gs_at<EQ, A>(F, i, j, k)) : "memory");
+    }
+  }
+}
+// the own field's staged registers into shared memory
+template <int EQ>
+__device__ __forceinline__ void gs_put(double *sm, int ch, const double *t) {
+  constexpr GsRows R = gs_rows<EQ>(0);
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < (R.n() + 3) / 4; ++q) {
+    const int r = 4 * q + lane / 8, i = kGsCh * ch + 2 - r % R.nj - r / R.nj + lane % 8;
+    if (r < R.n()) sm[r * kGsPitch + (i & (kGsRing - 1))] = t[q];
+  }
+}
+
+// Sweep n of the window on tile (J, K); returns this lane's residual sum.
+// sm: the warp's staged rows.
+template <int EQ>
+__device__ double gs_tile(const FluidDev &F, const Prm &P, double *own, double *sm, int J, int K, int nJ, int nK, int NI,
+                          int NJ, int NK, int n, int nch, bool lid, GsFlags &fl) {
+  const int lane = threadIdx.x & 31, jj = lane % kTJ, kk = lane / kTJ;
+  const int j0 = J * kTJ + 1, k0 = K * kTK + 1, j = j0 + jj, k = k0 + kk, off = jj + kk;
+  const int tile = J + nJ * K;
+  const bool row = j <= NJ && k <= NK;
+  double *ap_out = EQ == 0 ? F.up : EQ == 1 ? F.vp : F.wp;
+  // the tiles this one waits for: (J-1, K) and (J, K-1) in this sweep, (J+1, K) and (J, K+1) in the one before
+  int idx = -1;
+  if (lane == 0 && J > 0) idx = tile - 1;
+  if (lane == 1 && K > 0) idx = tile - nJ;
+  if (lane == 2 && n > 0 && J + 1 < nJ) idx = tile + 1;
+  if (lane == 3 && n > 0 && K + 1 < nK) idx = tile + nJ;
+  const int base = (lane < 2 ? n : n - 1) * nch;
+  // Chunk ch takes new values of (J-1, K) up to its step kGsCh (ch + 1) - 1 + 7
+  // and of (J, K-1) up to + 3, and stages, for the chunk after it, old values
+  // of (J+1, K) and (J, K+1) up to their steps kGsCh (ch + 2) - 8 and - 4: within
+  // chunk ch + 1 of each
+  static_assert(kTJ - 1 <= kGsCh && kTK <= kGsCh && kTJ <= kGsCh, "chunk lag");
+  constexpr int NT = (gs_rows<EQ>(0).n() + 3) / 4;
+  double t[NT];
+  uint8_t em[kGsCh];
+  unsigned en = 0u;
+  double *sg = sm + gs_base<EQ>(4) * kGsPitch;
+  auto stage = [&](int ch) {
+    gs_stage<EQ, 0>(F, sm, ch, j0, k0, NI, NJ, NK, t);
+    gs_stage<EQ, 1>(F, sm, ch, j0, k0, NI, NJ, NK, t);
+    gs_stage<EQ, 2>(F, sm, ch, j0, k0, NI, NJ, NK, t);
+    gs_stage<EQ, 3>(F, sm, ch, j0, k0, NI, NJ, NK, t);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {  // x geometry, eight lanes an array
+      const int a = 4 * q + lane / 8, i = kGsCh * ch + 2 + lane % 8;
+      if (a < (EQ == 3 ? 4 : 5) && i >= 0 && i <= NI + 1) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(sg + a * kGsPitch + (i & (kGsRing - 1)));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gs_geo<EQ>(F, a) + i) : "memory");
+      }
+    }
+    // the masks of this lane's cells of the chunk (bit q: not fluid)
+    en = 0u;
+#pragma unroll
+    for (int q = 0; q < kGsCh; ++q) {
+      const int i = ch * kGsCh + q - off + 1;
+      em[q] = row && i >= 1 && i <= NI ? __ldg(F.empty + GC(F, i - 1, j - 1, k - 1)) : (uint8_t)0;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto staged = [&](int ch) {
+    gs_put<EQ>(sm, ch, t);
+#pragma unroll
+    for (int q = 0; q < kGsCh; ++q) en |= em[q] ? 1u << q : 0u;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+  };
+  __syncwarp();  // the tile before has read its rows
+  if (n > 0) fl.wait(idx, base + min(nch, 2));  // the first sweep's old values are there from the start
+  stage(-1);
+  staged(-1);
+  stage(0);
+  staged(0);
+  if (n == 0) fl.wait(idx, base + min(nch, 2));
+  // this lane's rows in the staged arrays
+  const double *so = sm + (jj + (kTJ + 1) * kk) * kGsPitch;
+  auto xrow = [&](int a, int dj, int dk) {
+    const GsRows R = gs_rows<EQ>(a);
+    return sm + (gs_base<EQ>(a) + (jj + dj - R.dj) + R.nj * (kk + dk - R.dk)) * kGsPitch;
+  };
+  double res = 0.0, acc = 0.0;
+  const bool eJ = row && jj == 0, eK = row && kk == 0;
+  for (int ch = 0; ch < nch; ++ch) {
+    if (ch > 0) fl.wait(idx, base + min(nch, ch + 2));
+    // the new values below the tile's lower edges, for the whole chunk
+    double sJ[kGsCh], sK[kGsCh];
+#pragma unroll
+    for (int q = 0; q < kGsCh; ++q) {
+      const int i = ch * kGsCh + q - off + 1;
+      const bool in = i >= 1 && i <= NI;
+      sJ[q] = eJ && in ? ld(own + gs_idx<EQ>(F, i, j - 1, k)) : 0.0;
+      sK[q] = eK && in ? ld(own + gs_idx<EQ>(F, i, j, k - 1)) : 0.0;
+    }
+    const unsigned mask = en;
+    if (ch + 1 < nch) stage(ch + 1);
+#pragma unroll
+    for (int q = 0; q < kGsCh; ++q) {
+      const int i = ch * kGsCh + q - off + 1;
+      // res: the value this lane left at the step before
+      const double fj = __shfl_up_sync(0xffffffffu, res, 1), fk = __shfl_up_sync(0xffffffffu, res, kTJ);
+      if (row && i >= 1 && i <= NI) {
+        const bool empty = mask >> q & 1u;
+        const int r0 = i & (kGsRing - 1), rp = (i + 1) & (kGsRing - 1), rm = (i - 1) & (kGsRing - 1);
+        GsIn<EQ> in;
+        in.c = so[r0];
+        in.e = so[rp];
+        in.n = so[kGsPitch + r0];
+        in.b = so[(kTJ + 1) * kGsPitch + r0];
+#pragma unroll
+        for (int a = 0; a < (EQ == 3 ? 4 : 5); ++a) in.g[a] = sg[a * kGsPitch + r0];
+        if constexpr (EQ == 0) {
+          in.x[0] = xrow(1, 0, 0)[r0]; in.x[1] = xrow(1, 1, 0)[r0]; in.x[2] = xrow(2, 0, 0)[r0]; in.x[3] = xrow(2, 0, 1)[r0];
+          in.x[4] = xrow(3, 0, 0)[r0];
+          in.cx[0] = xrow(1, 0, 0)[rm]; in.cx[1] = xrow(1, 1, 0)[rm]; in.cx[2] = xrow(2, 0, 0)[rm]; in.cx[3] = xrow(2, 0, 1)[rm];
+          in.cx[4] = xrow(3, 0, 0)[rm];
+        } else if constexpr (EQ == 1) {
+          in.x[0] = xrow(1, 0, 0)[rp]; in.x[1] = xrow(1, -1, 0)[rp]; in.cx[0] = xrow(1, 0, 0)[r0]; in.cx[1] = xrow(1, -1, 0)[r0];
+          in.x[2] = xrow(2, 0, 1)[r0]; in.x[3] = xrow(2, -1, 1)[r0]; in.x[4] = xrow(2, 0, 0)[r0]; in.x[5] = xrow(2, -1, 0)[r0];
+          in.x[6] = xrow(3, -1, 0)[r0]; in.x[7] = xrow(3, 0, 0)[r0];
+        } else if constexpr (EQ == 2) {
+          in.x[0] = xrow(1, 0, 0)[rp]; in.x[1] = xrow(1, 0, -1)[rp]; in.cx[0] = xrow(1, 0, 0)[r0]; in.cx[1] = xrow(1, 0, -1)[r0];
+          in.x[2] = xrow(2, 0, 0)[r0]; in.x[3] = xrow(2, 0, -1)[r0]; in.x[4] = xrow(2, 1, 0)[r0]; in.x[5] = xrow(2, 1, -1)[r0];
+          in.x[6] = xrow(3, 0, -1)[r0]; in.x[7] = xrow(3, 0, 0)[r0];
+        } else {
+          in.x[0] = xrow(1, 0, 0)[r0]; in.x[1] = xrow(2, 0, 0)[r0]; in.x[2] = xrow(3, 0, 0)[r0];
+        }
+        double ap = 0.0;
+        const double nv = gs_update<EQ>(F, P, i, j, k, i == 1 ? so[rm] : res, jj == 0 ? sJ[q] : fj, kk == 0 ? sK[q] : fk,
+                                        in, lid, ap);
+        if (!empty) {
+          const int e = gs_idx<EQ>(F, i, j, k);
+          own[e] = nv;
+          if (EQ != 3) ap_out[e] = ap;
+          acc += (nv - in.c) * (nv - in.c);
+        }
+        res = empty ? in.c : nv;
+      }
+    }
+    if (ch + 1 < nch) staged(ch + 1);
+    fl.done(tile, n * nch + ch + 1);
+  }
+  return acc;
+}
+
+// One GS solve of equation EQ (0 u, 1 v, 2 w momentum; 3 fluid energy), as far
+// as its windows have at most kTileW sweeps; a larger one is left to
+// k_gs_planes.  prog: one counter per tile; slots: window residuals, one per
+// sweep and warp; give_up: set when a wait runs out (in host memory).
+template <int EQ>
+__global__ void __launch_bounds__(kGsT, 1) k_gs_tiles(FluidDev F, Prm P, double *slots, int *prog, int *give_up, DevStats *st, double *snap) {
+  cg::grid_group grid = cg::this_grid();
+  __shared__ double tot[kTileW];
+  const int NI = EQ == 0 ? F.fx - 1 : F.cx, NJ = EQ == 1 ? F.fy - 1 : F.cy, NK = EQ == 2 ? F.fz - 1 : F.cz;
+  const double d1 = EQ == 2 ? F.fz : F.cz, d2 = EQ == 1 ? F.fy : F.cy, d3 = EQ == 0 ? F.fx : F.cx;
+  const double tol = EQ == 3 ? P.energy_tol : P.mom_tol;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+  extern __shared__ __align__(16) double gs_dyn[];
+  double *sm = gs_dyn + (threadIdx.x >> 5) * (gs_base<EQ>(4) + kGsGeo) * kGsPitch;
+  const int wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = gridDim.x * (kGsT / 32);
+  double *own = EQ == 0 ? F.u : EQ == 1 ? F.v : EQ == 2 ? F.w : F.tt;
+  const long long nown = EQ == 0 ? (long long)(F.fx + 2) * (F.cy + 2) * (F.cz + 2)
+                       : EQ == 1 ? (long long)(F.cx + 2) * (F.fy + 2) * (F.cz + 2)
+                       : EQ == 2 ? (long long)(F.cx + 2) * (F.cy + 2) * (F.fz + 2)
+                                 : (long long)(F.cx + 2) * (F.cy + 2) * (F.cz + 2);
+  const bool lid_row = (F.oy - 1 + F.fy - 1 == F.Ny);
+  const int nJ = (NJ + kTJ - 1) / kTJ, nK = (NK + kTK - 1) / kTK, ntile = nJ * nK;
+  const int nch = (NI + kTJ + kTK - 2 + kGsCh - 1) / kGsCh;
+  GsFlags fl{prog, give_up, false};
+  const int pred = st->sweeps[EQ] > 0 ? st->sweeps[EQ] : 2;
+  double residual = 1.0, gres = 1.0;
+  int done = 0;
+  while (done < P.gs_max && !(gres < tol)) {
+    int W = done < pred ? pred - done : max(1, done);
+    W = min(W, min(P.gs_max - done, kBlock));
+    if (W > kTileW) break;
+    if (W > 1)
+      for (long long q = tid; q < nown; q += T) snap[q] = ld(own + q);
+    int runs = 0, stop = W;
+    double r_new = residual, g_new = gres;
+    for (;;) {
+      for (int q = tid; q < ntile; q += T) prog[q] = 0;
+      grid.sync();  // also: every block has read the prediction before thread 0 rewrites it
+      // a warp takes its tiles in order, sweep by sweep: what a tile waits for
+      // comes before it in every warp's order, so some warp can always go on
+      for (int n = 0; n < W; ++n) {
+        double acc = 0.0;
+        for (int t = wid; t < ntile; t += nw)
+          acc += gs_tile<EQ>(F, P, own, sm, t % nJ, t / nJ, nJ, nK, NI, NJ, NK, n, nch,
+                             EQ == 1 && lid_row && (done + n) >= 1, fl);
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) slots[(size_t)n * nw + wid] = acc;
+      }
+      grid.sync();
+      for (int n = threadIdx.x >> 5; n < W; n += kGsT / 32) {
+        double a = 0.0;
+        for (int q = lane; q < nw; q += 32) a += __ldcg(slots + (size_t)n * nw + q);
+        for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) tot[n] = a;
+      }
+      __syncthreads();
+      if (runs == 1) break;  // the rerun reproduces the first pass exactly
+      // replay the reference's stop test sweep by sweep
+      double r = residual, g = gres;
+      stop = W;
+      for (int c = 1; c <= W; ++c) {
+        r = (r + tot[c - 1]) / d1 / d2 / d3;
+        g = sqrt(r);
+        if (g < tol || done + c >= P.gs_max) { stop = c; break; }
+      }
+      r_new = r; g_new = g;
+      runs = 1;
+      if (stop == W) break;
+      for (long long q = tid; q < nown; q += T) own[q] = snap[q];
+      __syncthreads();  // every warp has read tot
+      W = stop;
+    }
+    done += stop;
+    residual = r_new;
+    gres = g_new;
+  }
+  const bool open = done < P.gs_max && !(gres < tol);
+  if (!open) {
+    if (EQ == 0) bc_x(F, tid, T);
+    else if (EQ == 1) bc_y(F, P, tid, T);
+    else if (EQ == 2) bc_z(F, tid, T);
+  }
+  if (tid == 0) {
+    st->gs_open = open;
+    if (open) { st->gs_done = done; st->gs_residual = residual; st->gs_res = gres; }
+    else { st->sweeps[EQ] = done; st->res[EQ] = gres; st->cum_sweeps[EQ] += done; }
+  }
+}
 
 __device__ __forceinline__ int pow2_at_least(int w) { int a = 1; while (a < w) a <<= 1; return a; }
 
@@ -405,9 +839,11 @@ __device__ __forceinline__ void energy_apply(const FluidDev &F, const Prm &P, co
   acc += (nv - e.tc) * (nv - e.tc);
 }
 
-// One GS solve of equation EQ (0 u, 1 v, 2 w momentum; 3 fluid energy).
+// The windows of equation EQ that k_gs_tiles left (more than kTileW sweeps):
+// one grid barrier per hyperplane, all sweeps of the window in flight.
 template <int EQ>
-__global__ void __launch_bounds__(kBlock, 2) k_gs(FluidDev F, Prm P, double *partials, DevStats *st, double *snap) {
+__global__ void __launch_bounds__(kBlock, 2) k_gs_planes(FluidDev F, Prm P, double *partials, DevStats *st, double *snap) {
+  if (st->gs_open == 0) return;  // k_gs_tiles finished the solve
   cg::grid_group grid = cg::this_grid();
   __shared__ double red[kBlock];
   __shared__ double tot[kBlock];
@@ -436,9 +872,9 @@ __global__ void __launch_bounds__(kBlock, 2) k_gs(FluidDev F, Prm P, double *par
   const bool lid_row = (F.oy - 1 + F.fy - 1 == F.Ny);
   int buf = 0;
   const int pred = st->sweeps[EQ] > 0 ? st->sweeps[EQ] : 2;
-  grid.sync();  // every block has read the prediction before thread 0 rewrites it
-  double residual = 1.0, gres = 1.0;
-  int done = 0;
+  double residual = st->gs_residual, gres = st->gs_res;
+  int done = st->gs_done;
+  grid.sync();  // every block has read the state before thread 0 rewrites it
   while (done < P.gs_max && !(gres < tol)) {
     int W = done < pred ? pred - done : max(1, done);
     W = min(W, min(P.gs_max - done, kBlock));
@@ -1356,7 +1792,15 @@ struct DeviceState {
             *ibw_face = nullptr;
   int nibu = 0, nibv = 0, nibw = 0;
   // cooperative grid sizes
-  int g_gs[4] = {0, 0, 0, 0}, g_pcorr = 0, tz = 16;
+  int g_gs[4] = {0, 0, 0, 0}, g_tiles[4] = {0, 0, 0, 0}, g_pcorr = 0, tz = 16;
+  int *gs_prog = nullptr;      // the wavefront tiles' progress
+  double *gs_slots = nullptr;  // window residuals per sweep and warp
+  int *gave_up = nullptr;      // pinned: a wait between tiles ran out
+  // after the stream has been waited for
+  void check_waits() const {
+    if (*(volatile int *)gave_up)
+      throw std::runtime_error("Gauss-Seidel sweep: a wait between tiles ran out (the sweep was abandoned)");
+  }
   // optional per-phase CUDA-event timing on the engine stream
   bool profiling = false;
   std::vector<cudaEvent_t> ev_pool;
@@ -1400,6 +1844,7 @@ struct DeviceState {
     for (auto e : ev_pool) cudaEventDestroy(e);
     for (void *p : allocs) cudaFree(p);
     if (stats_host) cudaFreeHost(stats_host);
+    if (gave_up) cudaFreeHost(gave_up);
     if (stream) cudaStreamDestroy(stream);
   }
 };
@@ -1431,10 +1876,13 @@ int choose_tz(long cx, long cy, long cz, int grid) {
 }
 
 template <class K, class... A>
-void coop_launch(K kernel, int blocks, cudaStream_t s, A... args) {
+void coop_launch(K kernel, int blocks, int threads, int smem, cudaStream_t s, A... args) {
   void *argv[] = {(void *)&args...};
-  HS_CUDA(cudaLaunchCooperativeKernel((void *)kernel, dim3(blocks), dim3(kBlock), argv, 0, s));
+  HS_CUDA(cudaLaunchCooperativeKernel((void *)kernel, dim3(blocks), dim3(threads), argv, smem, s));
 }
+
+// tiles of the wavefront sweeps over nj x nk rows
+long gs_tiles(long nj, long nk) { return ((nj + kTJ - 1) / kTJ) * ((nk + kTK - 1) / kTK); }
 
 int grid_for(long n) { return (int)std::max<long>(1, std::min<long>((n + kBlock - 1) / kBlock, 148L * 16)); }
 
@@ -1589,10 +2037,27 @@ Engine::Engine(const Case &c, const hs_params &p, int device) : case_(c), prm_(p
   // cooperative grid sizes
   {
     long rows[4] = {M.cy * M.cz, (M.fy - 1) * M.cz, M.cy * (M.fz - 1), M.cy * M.cz};
-    D.g_gs[0] = coop_blocks(k_gs<0>, D.nsm, (int)std::min<long>((rows[0] + 1) / 2, 1 << 20));
-    D.g_gs[1] = coop_blocks(k_gs<1>, D.nsm, (int)std::min<long>((rows[1] + 1) / 2, 1 << 20));
-    D.g_gs[2] = coop_blocks(k_gs<2>, D.nsm, (int)std::min<long>((rows[2] + 1) / 2, 1 << 20));
-    D.g_gs[3] = coop_blocks(k_gs<3>, D.nsm, (int)std::min<long>((rows[3] + 1) / 2, 1 << 20));
+    D.g_gs[0] = coop_blocks(k_gs_planes<0>, D.nsm, (int)std::min<long>((rows[0] + 1) / 2, 1 << 20));
+    D.g_gs[1] = coop_blocks(k_gs_planes<1>, D.nsm, (int)std::min<long>((rows[1] + 1) / 2, 1 << 20));
+    D.g_gs[2] = coop_blocks(k_gs_planes<2>, D.nsm, (int)std::min<long>((rows[2] + 1) / 2, 1 << 20));
+    D.g_gs[3] = coop_blocks(k_gs_planes<3>, D.nsm, (int)std::min<long>((rows[3] + 1) / 2, 1 << 20));
+    // a warp per tile while the tiles' warps are resident at once, one warp per SM before a second
+    const long tiles[4] = {gs_tiles(M.cy, M.cz), gs_tiles(M.fy - 1, M.cz), gs_tiles(M.cy, M.fz - 1), gs_tiles(M.cy, M.cz)};
+    const void *ks[4] = {(const void *)k_gs_tiles<0>, (const void *)k_gs_tiles<1>, (const void *)k_gs_tiles<2>, (const void *)k_gs_tiles<3>};
+    const int sm[4] = {gs_smem<0>(), gs_smem<1>(), gs_smem<2>(), gs_smem<3>()};
+    long wmax = 1, tmax = 1;
+    for (int e = 0; e < 4; ++e) {
+      int per = 0;
+      HS_CUDA(cudaFuncSetAttribute(ks[e], cudaFuncAttributeMaxDynamicSharedMemorySize, sm[e]));
+      HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ks[e], kGsT, sm[e]));
+      if (per < 1) throw std::runtime_error("cooperative kernel cannot be resident");
+      const long one = std::min<long>(tiles[e], D.nsm);  // blocks of four warps
+      D.g_tiles[e] = (int)std::max<long>(1, tiles[e] <= one * (kGsT / 32) ? one : std::min<long>((long)per * D.nsm, (tiles[e] + kGsT / 32 - 1) / (kGsT / 32)));
+      wmax = std::max<long>(wmax, (long)D.g_tiles[e] * (kGsT / 32));
+      tmax = std::max(tmax, tiles[e]);
+    }
+    D.gs_prog = D.alloc<int>(tmax);
+    D.gs_slots = D.alloc<double>((size_t)kTileW * wmax);
   }
   D.g_pcorr = coop_blocks(k_pcorr, D.nsm, 1 << 30);
   D.tz = choose_tz(M.cx, M.cy, M.cz, D.g_pcorr);
@@ -1629,6 +2094,8 @@ Engine::Engine(const Case &c, const hs_params &p, int device) : case_(c), prm_(p
   D.stats = D.alloc<DevStats>(1);
   HS_CUDA(cudaMallocHost(&D.stats_host, sizeof(DevStats)));
   std::memset(D.stats_host, 0, sizeof(DevStats));
+  HS_CUDA(cudaMallocHost(&D.gave_up, sizeof(int)));
+  *D.gave_up = 0;
   HS_CUDA(cudaStreamSynchronize(D.stream));
 }
 
@@ -1685,18 +2152,30 @@ void Engine::step(int nsteps) {
   };
   for (int it = 0; it < nsteps; ++it) {
     // FluidSolver::solve (fluid_solver.h:1401-1633)
-    { Mark m(D, 0); coop_launch(k_gs<0>, D.g_gs[0], s, D.F, D.P, D.partials, D.stats, D.snap); }
-    { Mark m(D, 1); coop_launch(k_gs<1>, D.g_gs[1], s, D.F, D.P, D.partials, D.stats, D.snap); }
-    { Mark m(D, 2); coop_launch(k_gs<2>, D.g_gs[2], s, D.F, D.P, D.partials, D.stats, D.snap); }
+    {
+      Mark m(D, 0);
+      coop_launch(k_gs_tiles<0>, D.g_tiles[0], kGsT, gs_smem<0>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.stats, D.snap);
+      coop_launch(k_gs_planes<0>, D.g_gs[0], kBlock, 0, s, D.F, D.P, D.partials, D.stats, D.snap);
+    }
+    {
+      Mark m(D, 1);
+      coop_launch(k_gs_tiles<1>, D.g_tiles[1], kGsT, gs_smem<1>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.stats, D.snap);
+      coop_launch(k_gs_planes<1>, D.g_gs[1], kBlock, 0, s, D.F, D.P, D.partials, D.stats, D.snap);
+    }
+    {
+      Mark m(D, 2);
+      coop_launch(k_gs_tiles<2>, D.g_tiles[2], kGsT, gs_smem<2>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.stats, D.snap);
+      coop_launch(k_gs_planes<2>, D.g_gs[2], kBlock, 0, s, D.F, D.P, D.partials, D.stats, D.snap);
+    }
     int assemble = (!D.have_matrix || !prm_.frozen_matrix) ? 1 : 0;
     if (prm_.pressure_solver == HS_PSOLVE_MGCG) {
       Mark m(D, 3);
       k_pcorr_setup<<<grid_for(n), kBlock, 0, s>>>(D.F, assemble);
       if (assemble) build_multigrid();
-      coop_launch(k_mgcg, D.g_mgcg, s, D.F, D.P, D.mg, D.partials, D.stats);
+      coop_launch(k_mgcg, D.g_mgcg, kBlock, 0, s, D.F, D.P, D.mg, D.partials, D.stats);
     } else {
       Mark m(D, 3);
-      coop_launch(k_pcorr, D.g_pcorr, s, D.F, D.P, D.partials, D.stats, assemble, D.tz);
+      coop_launch(k_pcorr, D.g_pcorr, kBlock, 0, s, D.F, D.P, D.partials, D.stats, assemble, D.tz);
     }
     D.have_matrix = true;
     {
@@ -1704,11 +2183,15 @@ void Engine::step(int nsteps) {
       k_correct<<<grid_for(n), kBlock, 0, s>>>(D.F, D.P);
       HS_CUDA(cudaMemsetAsync(D.F.x, 0, sizeof(double) * (size_t)case_.fluid.npad(), s));
     }
-    { Mark m(D, 5); coop_launch(k_gs<3>, D.g_gs[3], s, D.F, D.P, D.partials, D.stats, D.snap); }
+    {
+      Mark m(D, 5);
+      coop_launch(k_gs_tiles<3>, D.g_tiles[3], kGsT, gs_smem<3>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.stats, D.snap);
+      coop_launch(k_gs_planes<3>, D.g_gs[3], kBlock, 0, s, D.F, D.P, D.partials, D.stats, D.snap);
+    }
     // MobSolver::solve for every region
     if (D.nreg) {
       Mark m(D, 6);
-      coop_launch(k_solid, D.solid_blocks, s, (const SolidReg *)D.regs, D.nreg, (const int *)D.blk_reg, D.stt, D.stc,
+      coop_launch(k_solid, D.solid_blocks, kBlock, 0, s, (const SolidReg *)D.regs, D.nreg, (const int *)D.blk_reg, D.stt, D.stc,
                   (const uint8_t *)D.sem, D.P, D.partials, D.stats, D.ssnap, D.spred);
     }
     {
@@ -1828,6 +2311,7 @@ void Engine::build_multigrid() {
 void Engine::sync() {
   HS_CUDA(cudaSetDevice(device_));
   HS_CUDA(cudaStreamSynchronize(d_->stream));
+  d_->check_waits();
 }
 
 void Engine::stats(hs_stats *out) {
@@ -1835,6 +2319,7 @@ void Engine::stats(hs_stats *out) {
   HS_CUDA(cudaMemcpyAsync(D.stats_host, D.stats, sizeof(DevStats), cudaMemcpyDeviceToHost, D.stream));
   HS_CUDA(cudaStreamSynchronize(D.stream));
   const DevStats &h = *D.stats_host;
+  D.check_waits();
   out->sweeps_u = h.sweeps[0]; out->sweeps_v = h.sweeps[1]; out->sweeps_w = h.sweeps[2]; out->sweeps_t = h.sweeps[3];
   out->sweeps_solid_max = h.solid_sweeps_max; out->pcg_iters = h.pcg_iters;
   out->res_u = h.res[0]; out->res_v = h.res[1]; out->res_w = h.res[2]; out->res_t = h.res[3];
@@ -1880,6 +2365,7 @@ void Engine::get_field(int f, double *host, long n) {
   if (!p || m != n) throw std::invalid_argument("field id or size mismatch");
   HS_CUDA(cudaMemcpyAsync(host, p, sizeof(double) * n, cudaMemcpyDeviceToHost, d_->stream));
   HS_CUDA(cudaStreamSynchronize(d_->stream));
+  d_->check_waits();
 }
 
 void Engine::set_field(int f, const double *host, long n) {
@@ -1902,6 +2388,7 @@ void Engine::get_solid(int r, int which, double *host, long n) {
   const double *src = which == 0 ? D.stt + R.tt_off : D.stc + R.tc_off;
   HS_CUDA(cudaMemcpyAsync(host, src, sizeof(double) * n, cudaMemcpyDeviceToHost, D.stream));
   HS_CUDA(cudaStreamSynchronize(D.stream));
+  D.check_waits();
 }
 
 // ---------------------------------------------------------------- standalone CG
@@ -1953,7 +2440,7 @@ void pcg_solve(PcgWork *w, const double *acx, const double *acy, const double *a
   HS_CUDA(cudaSetDevice(w->device));
   cudaStream_t st = (cudaStream_t)stream;
   CgView V{w->cx, w->cy, w->cz, acx, acy, acz, x, w->r, w->pa, w->pb, w->s};
-  coop_launch(k_pcg, w->grid, st, V, b, tol, maxiter, w->partials, w->tz, w->iters, w->relres);
+  coop_launch(k_pcg, w->grid, kBlock, 0, st, V, b, tol, maxiter, w->partials, w->tz, w->iters, w->relres);
   int it = 0;
   double rr = 0;
   HS_CUDA(cudaMemcpyAsync(&it, w->iters, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -2036,7 +2523,7 @@ void pcg_solve_noalloc(int nx, int ny, int nz, const double *acx, const double *
   // k_pcg writes every scratch word it later reads (r, p, s over the padded
   // grid, each partial before its reduction, both results), so the previous
   // call's contents never leak into this one
-  coop_launch(k_pcg, S.grid, st, V, b, tol, maxiter, partials, choose_tz(nx, ny, nz, S.grid), out_it, out_rel);
+  coop_launch(k_pcg, S.grid, kBlock, 0, st, V, b, tol, maxiter, partials, choose_tz(nx, ny, nz, S.grid), out_it, out_rel);
   int it = 0;
   double rr = 0;
   HS_CUDA(cudaMemcpyAsync(&it, out_it, sizeof(int), cudaMemcpyDeviceToHost, st));
