@@ -90,7 +90,7 @@ struct DevStats {
   int pcg_iters;
   double pcg_relres;
   int solid_sweeps_max;
-  int pad;
+  int gave_up;        // a wait of k_gs_tiles ran out
   // the solve that k_gs_tiles leaves to k_gs_planes: its sweeps and residuals so far
   int gs_open, gs_done;
   double gs_residual, gs_res;
@@ -479,7 +479,7 @@ __device__ __forceinline__ double gs_update(const FluidDev &F, const Prm &P, int
 // A warp's view of the tiles' progress (chunks finished, counted over the sweeps of the window)
 struct GsFlags {
   int *prog;       // one per tile
-  int *give_up;    // set by the first wait that runs out; no wait is taken after it
+  int *give_up, *told;  // set by the first wait that runs out (device, host memory); no wait is taken after it
   bool dead;
   // lanes 0..3 hold one tile index and the count it must have reached (idx < 0: none)
   __device__ __forceinline__ void wait(int idx, int need) {
@@ -495,7 +495,7 @@ struct GsFlags {
           break;
         }
       }
-      if (dead && (threadIdx.x & 31) == 0) *(volatile int *)give_up = 1;
+      if (dead && (threadIdx.x & 31) == 0) *(volatile int *)give_up = *(volatile int *)told = 1;
     }
     __syncwarp();
   }
@@ -677,9 +677,9 @@ __device__ double gs_tile(const FluidDev &F, const Prm &P, double *own, double *
 // One GS solve of equation EQ (0 u, 1 v, 2 w momentum; 3 fluid energy), as far
 // as its windows have at most kTileW sweeps; a larger one is left to
 // k_gs_planes.  prog: one counter per tile; slots: window residuals, one per
-// sweep and warp; give_up: set when a wait runs out (in host memory).
+// sweep and warp; told: set when a wait runs out (host memory: not for polling).
 template <int EQ>
-__global__ void __launch_bounds__(kGsT, 1) k_gs_tiles(FluidDev F, Prm P, double *slots, int *prog, int *give_up, DevStats *st, double *snap) {
+__global__ void __launch_bounds__(kGsT, 1) k_gs_tiles(FluidDev F, Prm P, double *slots, int *prog, int *told, DevStats *st, double *snap) {
   cg::grid_group grid = cg::this_grid();
   __shared__ double tot[kTileW];
   const int NI = EQ == 0 ? F.fx - 1 : F.cx, NJ = EQ == 1 ? F.fy - 1 : F.cy, NK = EQ == 2 ? F.fz - 1 : F.cz;
@@ -698,7 +698,7 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_tiles(FluidDev F, Prm P, double 
   const bool lid_row = (F.oy - 1 + F.fy - 1 == F.Ny);
   const int nJ = (NJ + kTJ - 1) / kTJ, nK = (NK + kTK - 1) / kTK, ntile = nJ * nK;
   const int nch = (NI + kTJ + kTK - 2 + kGsCh - 1) / kGsCh;
-  GsFlags fl{prog, give_up, false};
+  GsFlags fl{prog, &st->gave_up, told, false};
   const int pred = st->sweeps[EQ] > 0 ? st->sweeps[EQ] : 2;
   double residual = 1.0, gres = 1.0;
   int done = 0;
