@@ -81,6 +81,9 @@ struct FluidDev {
 
 struct SolidReg {
   int cx, cy, cz, rows, blk0, nblk;
+  int id;              // region number
+  int nlist;           // k_solid_block: non-empty cells
+  long long hyp_off;   // and the start of its hyperplane offsets
   long long tt_off, tc_off, em_off;
 };
 
@@ -968,7 +971,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_gs_planes(FluidDev F, Prm P, doub
 constexpr int kMaxRegions = 256;
 __global__ void __launch_bounds__(kBlock, 2) k_solid(const SolidReg *regs, int nreg, const int *blk_reg, double *tt_all,
                                                   double *tc_all, const uint8_t *em_all, Prm P, double *partials,
-                                                  DevStats *st, double *snap, int *pred_all) {
+                                                  double *snap, int *pred_all) {
   cg::grid_group grid = cg::this_grid();
   __shared__ double red[kBlock];
   __shared__ double r2[kMaxRegions];
@@ -994,7 +997,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_solid(const SolidReg *regs, int n
         const bool act = done[q] < P.gs_max && !(r2[q] < P.solid_tol);
         int w = 0;
         if (act) {
-          const int pr = pred_all[q] > 0 ? pred_all[q] : 2;
+          const int pr = pred_all[regs[q].id] > 0 ? pred_all[regs[q].id] : 2;
           w = done[q] < pr ? pr - done[q] : max(1, done[q]);
           w = min(w, min(P.gs_max - done[q], kBlock));
           any = 1;
@@ -1107,23 +1110,122 @@ __global__ void __launch_bounds__(kBlock, 2) k_solid(const SolidReg *regs, int n
     __syncthreads();
   }
   grid.sync();  // every block has read pred_all before it is rewritten
-  if (blockIdx.x == 0) {
-    for (int q = threadIdx.x; q < nreg; q += blockDim.x) pred_all[q] = done[q];
-    if (threadIdx.x == 0) {
-      int m = 0;
-      long long cells = 0;
-      for (int q = 0; q < nreg; ++q) {
-        m = max(m, done[q]);
-        cells += (long long)done[q] * regs[q].cx * regs[q].cy * regs[q].cz;
+  if (blockIdx.x == 0)
+    for (int q = threadIdx.x; q < nreg; q += blockDim.x) pred_all[regs[q].id] = done[q];
+}
+
+// The same for a region whose box fits in one SM's shared memory, by one
+// block: every step of the wavefront is then a block barrier and shared-memory
+// loads instead of a grid barrier and a trip to L2.  At step t sweep n is on
+// hyperplane t - 2 n; a warp takes whole hyperplanes, whose cells are listed
+// (hyperplane by hyperplane, without the empty cells) when the region is set
+// up, so its lanes are full and one warp sum per hyperplane gives the sweep's
+// residual in a fixed order.  Bound by shared-memory loads: seven 8-byte
+// values per update.
+constexpr int kSolidT = 1024, kSolidW = 128;  // threads, sweeps per window
+inline __host__ __device__ int solid_px(int cx) { return (cx + 3) & ~1; }  // even: the lanes' stride along a hyperplane is odd
+inline __host__ __device__ long long solid_smem(int cx, int cy, int cz) {
+  return 8LL * solid_px(cx) * (cy + 2) * (cz + 2) + 4LL * (cx + cy + cz) + 2LL * cx * cy * cz;
+}
+constexpr long long kSolidSmem = 224 * 1024;
+
+__global__ void __launch_bounds__(kSolidT, 1) k_solid_block(const SolidReg *regs, const int *hyp_all,
+                                                            const uint16_t *list_all, double *tt_all, double *tc_all,
+                                                            Prm P, double *snap, int *pred_all) {
+  extern __shared__ __align__(16) double sol_sm[];
+  __shared__ double tot[kSolidW];
+  const SolidReg R = regs[blockIdx.x];
+  const int cx = R.cx, cy = R.cy, cz = R.cz, GX = cx + 2, PX = solid_px(cx), PXY = PX * (cy + 2);
+  const int npad = GX * (cy + 2) * (cz + 2), S = cx + cy + cz - 2;
+  double *T = sol_sm;
+  int *hyp = reinterpret_cast<int *>(T + (size_t)PXY * (cz + 2));  // first list entry of each hyperplane, S + 1
+  uint16_t *list = reinterpret_cast<uint16_t *>(hyp + S + 2);
+  double *G = tt_all + R.tt_off, *snp = snap + R.tt_off;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto at = [&](int q) { return q + (q / GX) * (PX - GX); };  // padded index in shared memory
+  for (int c = tid; c <= S; c += kSolidT) hyp[c] = hyp_all[R.hyp_off + c];
+  for (int c = tid; c < R.nlist; c += kSolidT) list[c] = list_all[R.em_off + c];
+  // applyOuterBoundaryCondition: every cell of the box to T1 (mobs_solver.h:105-115)
+  for (int c = tid; c < cx * cy * cz; c += kSolidT) tc_all[R.tc_off + c] = P.t_solid0;
+  for (int q = tid; q < npad; q += kSolidT) T[at(q)] = G[q];
+  const int pred = pred_all[R.id] > 0 ? pred_all[R.id] : 2;
+  __syncthreads();  // every thread has read the prediction before it is rewritten
+  double r2 = 1.0;
+  int done = 0;
+  while (done < P.gs_max && !(r2 < P.solid_tol)) {
+    int W = done < pred ? pred - done : max(1, done);
+    W = min(W, min(P.gs_max - done, kSolidW));
+    if (W > 1)
+      for (int q = tid; q < npad; q += kSolidT) snp[q] = T[at(q)];
+    int stop = W;
+    double rnew = r2;
+    for (int run = 0; run < 2; ++run) {
+      for (int n = tid; n < W; n += kSolidT) tot[n] = 0.0;
+      __syncthreads();
+      for (int t = 0; t < S + 2 * (W - 1); ++t) {
+        // sweeps nhi, nhi - 1, ... are on hyperplanes t - 2 nhi, t - 2 nhi + 2, ...
+        const int nhi = min(t >> 1, W - 1);
+        for (int n = nhi - warp; n >= 0 && t - 2 * n < S; n -= kSolidT / 32) {
+          const int c1 = hyp[t - 2 * n + 1];
+          double acc = 0.0;
+          for (int c = hyp[t - 2 * n] + lane; c < c1; c += 64) {
+            // two of the hyperplane's cells (independent of one another), every load before a store
+            const bool two = c + 32 < c1;
+            double *q = T + list[c], *u = T + list[two ? c + 32 : c];
+            const double old = q[0], ol2 = u[0];
+            double nv = 1.0 / 6.0 * (q[1] + q[-1] + q[-PX] + q[PX] + q[-PXY] + q[PXY]);
+            double nv2 = 1.0 / 6.0 * (u[1] + u[-1] + u[-PX] + u[PX] + u[-PXY] + u[PXY]);
+            nv = nv * P.relax_solid + (1 - P.relax_solid) * old;
+            nv2 = nv2 * P.relax_solid + (1 - P.relax_solid) * ol2;
+            *q = nv;
+            acc += (nv - old) * (nv - old);
+            if (two) {
+              *u = nv2;
+              acc += (nv2 - ol2) * (nv2 - ol2);
+            }
+          }
+          for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+          if (lane == 0) tot[n] += acc;
+        }
+        __syncthreads();
       }
-      st->solid_sweeps_max = m;
-      st->cum_solid_cell_sweeps += cells;
+      if (run == 1) break;
+      // the reference's stop test, sweep by sweep (mobs_solver.h:303-319)
+      double r = r2;
+      for (int c = 1; c <= W; ++c) {
+        r = sqrt((r + tot[c - 1]) / (double)cz / (double)cy / (double)cx);
+        if (r < P.solid_tol || done + c >= P.gs_max) { stop = c; break; }
+      }
+      rnew = r;
+      if (stop == W) break;
+      // overran: restore and rerun exactly `stop` sweeps
+      for (int q = tid; q < npad; q += kSolidT) T[at(q)] = snp[q];
+      W = stop;
+      __syncthreads();
     }
+    done += stop;
+    r2 = rnew;
+    __syncthreads();
   }
+  for (int q = tid; q < npad; q += kSolidT) G[q] = T[at(q)];
+  if (tid == 0) pred_all[R.id] = done;
 }
 
 // MobSolver::setForNext (mobs_solver.h:290-301)
-__global__ void k_solid_setfornext(const SolidReg *regs, int nreg, double *tt_all, double *tc_all, const uint8_t *em_all) {
+// and the statistics of the solid solves, whose sweeps are in pred_all
+__global__ void k_solid_setfornext(const SolidReg *regs, int nreg, double *tt_all, double *tc_all, const uint8_t *em_all,
+                                   const int *pred_all, DevStats *st) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    int m = 0;
+    long long cells = 0;
+    for (int q = 0; q < nreg; ++q) {
+      const int n = pred_all[regs[q].id];
+      m = max(m, n);
+      cells += (long long)n * regs[q].cx * regs[q].cy * regs[q].cz;
+    }
+    st->solid_sweeps_max = m;
+    st->cum_solid_cell_sweeps += cells;
+  }
   for (int r = blockIdx.y; r < nreg; r += gridDim.y) {
     const SolidReg R = regs[r];
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < R.cx * R.cy * R.cz; c += gridDim.x * blockDim.x) {
@@ -1777,7 +1879,10 @@ struct DeviceState {
   DevStats *stats_host = nullptr;
   // solids
   int nreg = 0, solid_blocks = 0, maxS = 0;
-  SolidReg *regs = nullptr;
+  int nsol_block = 0, nsol_coop = 0, sol_smem = 0;  // regions solved by one block each, by the cooperative kernel
+  SolidReg *regs = nullptr, *regs_block = nullptr, *regs_coop = nullptr;
+  int *sol_hyp = nullptr;        // k_solid_block: hyperplane offsets, cell lists
+  uint16_t *sol_list = nullptr;
   int *blk_reg = nullptr;
   std::vector<SolidReg> regs_h;
   double *stt = nullptr, *stc = nullptr;
@@ -1961,31 +2066,60 @@ Engine::Engine(const Case &c, const hs_params &p, int device) : case_(c), prm_(p
   std::vector<double> tt_h, tc_h;
   std::vector<uint8_t> em_h;
   D.regs_h.resize(D.nreg);
-  long long want_blocks = 0;
   for (int r = 0; r < D.nreg; ++r) {
     const Meta &S = c.solids[r];
     SolidReg &R = D.regs_h[r];
     R.cx = (int)S.cx; R.cy = (int)S.cy; R.cz = (int)S.cz; R.rows = (int)(S.cy * S.cz);
+    R.id = r;
     R.tt_off = (long long)tt_h.size(); R.tc_off = (long long)tc_h.size(); R.em_off = (long long)em_h.size();
     tt_h.insert(tt_h.end(), S.npad(), p.t_solid0);
     tc_h.insert(tc_h.end(), S.ncell(), 0.0);
     em_h.insert(em_h.end(), c.solid_empty[r].begin(), c.solid_empty[r].end());
     D.maxS = std::max<int>(D.maxS, (int)(S.cx + S.cy + S.cz - 2));
-    want_blocks += (R.rows + 1) / 2;
   }
   D.ntt = (long long)tt_h.size(); D.ntc = (long long)tc_h.size();
   D.stt = D.upload(tt_h); D.stc = D.upload(tc_h); D.sem = D.upload(em_h);
   if (D.nreg) {
+    // a region whose box fits in shared memory gets one block of its own
+    // (k_solid_block), the others share the cooperative kernel
+    std::vector<SolidReg> fits, rest;
+    for (const SolidReg &R : D.regs_h) (solid_smem(R.cx, R.cy, R.cz) <= kSolidSmem ? fits : rest).push_back(R);
+    std::vector<int> hyp;
+    std::vector<uint16_t> list(em_h.size(), 0);
+    for (SolidReg &R : fits) {
+      R.hyp_off = (long long)hyp.size();
+      R.nlist = 0;
+      const int px = solid_px(R.cx), pxy = px * (R.cy + 2);
+      for (int sp = 0; sp < R.cx + R.cy + R.cz - 2; ++sp) {
+        hyp.push_back(R.nlist);
+        for (int k = 0; k < R.cz; ++k)
+          for (int j = 0; j < R.cy; ++j) {
+            const int i = sp - j - k;
+            if (i < 0 || i >= R.cx || em_h[R.em_off + i + R.cx * (j + R.cy * k)]) continue;
+            list[R.em_off + R.nlist++] = (uint16_t)((i + 1) + px * (j + 1) + pxy * (k + 1));
+          }
+      }
+      hyp.push_back(R.nlist);
+    }
+    D.sol_hyp = D.upload(hyp);
+    D.sol_list = D.upload(list);
+    D.nsol_block = (int)fits.size();
+    for (const SolidReg &R : fits) D.sol_smem = std::max<int>(D.sol_smem, (int)solid_smem(R.cx, R.cy, R.cz));
+    if (D.nsol_block)
+      HS_CUDA(cudaFuncSetAttribute(k_solid_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolidSmem));
+    D.nsol_coop = (int)rest.size();
+    long long want_blocks = 0;
+    for (const SolidReg &R : rest) want_blocks += (R.rows + 1) / 2;
     int per = 0;
     HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_solid, kBlock, 0));
     long long cap = (long long)per * D.nsm;
-    if (cap < D.nreg) throw std::runtime_error("too many solid regions for one cooperative launch");
+    if (cap < D.nsol_coop) throw std::runtime_error("too many solid regions for one cooperative launch");
     std::vector<int> blk_reg;
     int b0 = 0;
-    for (int r = 0; r < D.nreg; ++r) {
-      SolidReg &R = D.regs_h[r];
+    for (int r = 0; r < D.nsol_coop; ++r) {
+      SolidReg &R = rest[r];
       long long wantr = (R.rows + 1) / 2;  // room for a 128-sweep window at 2 slots per thread
-      long long nb = want_blocks <= cap ? wantr : std::max<long long>(1, wantr * (cap - D.nreg) / want_blocks);
+      long long nb = want_blocks <= cap ? wantr : std::max<long long>(1, wantr * (cap - D.nsol_coop) / want_blocks);
       if (b0 + nb > cap) nb = 1;
       R.blk0 = b0; R.nblk = (int)nb;
       for (int q = 0; q < nb; ++q) blk_reg.push_back(r);
@@ -1993,6 +2127,8 @@ Engine::Engine(const Case &c, const hs_params &p, int device) : case_(c), prm_(p
     }
     D.solid_blocks = b0;
     D.regs = D.upload(D.regs_h);
+    D.regs_block = D.upload(fits);
+    D.regs_coop = D.upload(rest);
     D.blk_reg = D.upload(blk_reg);
   }
   // interface swap lists (solid indices made absolute into the joined buffer)
@@ -2191,8 +2327,12 @@ void Engine::step(int nsteps) {
     // MobSolver::solve for every region
     if (D.nreg) {
       Mark m(D, 6);
-      coop_launch(k_solid, D.solid_blocks, kBlock, 0, s, (const SolidReg *)D.regs, D.nreg, (const int *)D.blk_reg, D.stt, D.stc,
-                  (const uint8_t *)D.sem, D.P, D.partials, D.stats, D.ssnap, D.spred);
+      if (D.nsol_block)
+        k_solid_block<<<D.nsol_block, kSolidT, D.sol_smem, s>>>(D.regs_block, D.sol_hyp, D.sol_list, D.stt, D.stc, D.P,
+                                                                D.ssnap, D.spred);
+      if (D.nsol_coop)
+        coop_launch(k_solid, D.solid_blocks, kBlock, 0, s, (const SolidReg *)D.regs_coop, D.nsol_coop,
+                    (const int *)D.blk_reg, D.stt, D.stc, (const uint8_t *)D.sem, D.P, D.partials, D.ssnap, D.spred);
     }
     {
       Mark m(D, 7);
@@ -2206,7 +2346,7 @@ void Engine::step(int nsteps) {
       k_cellbc_resolve<<<grid_for(n), kBlock, 0, s>>>(D.F);
       k_cellbc_commit<<<grid_for(n), kBlock, 0, s>>>(D.F, D.P, 1);
       // MobSolver::setForNext
-      if (D.nreg) k_solid_setfornext<<<dim3(64, std::min(D.nreg, 64)), kBlock, 0, s>>>(D.regs, D.nreg, D.stt, D.stc, D.sem);
+      if (D.nreg) k_solid_setfornext<<<dim3(64, std::min(D.nreg, 64)), kBlock, 0, s>>>(D.regs, D.nreg, D.stt, D.stc, D.sem, D.spred, D.stats);
     }
     HS_CUDA(cudaGetLastError());
     steps_++;
