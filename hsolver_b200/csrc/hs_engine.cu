@@ -17,8 +17,10 @@
 // tol 1e-5, maxiter 1000, zero start; fluid_solver.h:1871-1875), run as one
 // cooperative kernel with two grid reductions per iteration.  The direction
 // update p = r + beta p is fused into the next SpMV (double-buffered p), and
-// x += alpha p is deferred into the same pass, so an iteration streams
-// r, p, x, 3 coefficients and writes p, s, x, then streams r, s and writes r.
+// x takes two directions at a time in the same pass of every other iteration,
+// so an iteration streams r, p, 3 coefficients and writes p, s (and in every
+// other one reads x and an older p and writes x), then streams r, s and
+// writes r: 92 B per cell.
 //
 // Reductions are deterministic: per-block partials, then every block sums
 // the partials in the same fixed order.
@@ -1255,14 +1257,23 @@ __global__ void k_swap_scatter(const long long *f_recv, const long long *s_recv,
 // ---------------------------------------------------------------- pressure correction
 // Assembly (fluid_solver.h:1969-2002 / 2123-2162) + HYPRE PCG restated.
 //
-// Pass A of an iteration (p = r + beta p, s = A p, x += alpha_prev p_old,
-// <s,p>) runs over 32 x 8 x TZ tiles: each block marches a tile column in
-// z, keeping three planes of the new direction (with a one-cell halo) in
-// shared memory, so every neighbour comes from shared memory and each cell's
-// r and p are read once.  Coefficients are zero off the fluid cells, where
-// r, p, x, s stay zero, so no mask test is needed.  Pass B (r -= alpha s,
-// <r,r>) streams the padded arrays as double2.
-constexpr int kTX = 32, kTY = 16;  // CG tiles of 32 x 16 columns; a thread owns rows ty and ty + 8
+// Pass A of an iteration (p = r + beta p, s = A p, <s,p>, and in every other
+// iteration x += the two directions before) runs over 32 x 16 x TZ tiles: a
+// thread group marches a tile column in z, keeping the last planes of the new
+// direction (with a one-cell halo) in shared memory, so every neighbour comes
+// from shared memory and each cell's r and p are read once.  Coefficients are
+// zero off the fluid cells, where r, p, x, s stay zero, so no mask test is
+// needed.  Pass B (r -= alpha s, <r,r>) streams the padded arrays as double2.
+constexpr int kTX = 32, kTY = 16, kTB = kTY / 2;  // CG tiles of 32 x 16 columns; a thread owns rows ty and ty + kTB
+static_assert(kTX * kTB == 256 && 2 * (kTX + kTY) <= 256, "a group's threads");
+// One block per SM, so that the grid barriers of an iteration have few
+// arrivals, of two groups of 256 threads (126 registers), each with tiles and
+// a named barrier of its own, and the loads of a plane issued a plane ahead.
+// Per iteration, against 256-thread blocks at the registers' occupancy
+// without loads ahead: 50x50x50 12.9 -> 9.9 us, 128^3 50.7 -> 41.4, 256x128x128
+// 97.5 -> 81.7 (one group 116, three or four spill).
+constexpr int kCgG = 2, kCgT = 256 * kCgG;
+constexpr int kCgSmem = kCgG * 4 * (kTY + 2) * (kTX + 2) * 8;
 
 // The CG iterations of hypre_PCGSolve restated (identity preconditioner,
 // two-norm test <r,r>/<b,b> < tol^2, maxiter): on entry r = p_a = b, x = 0 on
@@ -1275,64 +1286,85 @@ struct CgView {
 
 __device__ void cg_core(const CgView &V, double bb, double tol, int maxiter, double *partials, int &buf, double *sh,
                         cg::grid_group &grid, int TZ, int *out_iters, double *out_relres) {
-  __shared__ double pl[4][kTY + 2][kTX + 2];  // four plane slots: the plane written at kk never aliases those read at kk - 1
+  // four plane slots per group: the plane written at kk never aliases those read at kk - 1
+  extern __shared__ __align__(16) double cg_dyn[];
+  const int grp = threadIdx.x >> 8, gtid = threadIdx.x & 255;
+  double (*pl)[kTY + 2][kTX + 2] = reinterpret_cast<double (*)[kTY + 2][kTX + 2]>(cg_dyn) + 4 * grp;
+  auto group_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(grp + 1) : "memory"); };
   const int cx = V.cx, cy = V.cy, cz = V.cz;
   const int PX = cx + 2, PXY = (cx + 2) * (cy + 2);
   const long long npad = (long long)PXY * (cz + 2);
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
   const double eps = tol * tol;
-  double gamma = bb, iprod = bb, beta = 0.0, alpha_prev = 0.0, acc;
+  double gamma = bb, iprod = bb, beta = 0.0, alpha_prev = 0.0, alpha_prev2 = 0.0, acc;
   double *pold = V.pa, *pnew = V.pb;
   const int ntx = (cx + kTX - 1) / kTX, nty = (cy + kTY - 1) / kTY, ntz = (cz + TZ - 1) / TZ;
   const int ntiles = ntx * nty * ntz;
-  const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;  // ty in [0, 8)
-  // halo role (96 cells: y-1 row, y+16 row, x-1 column, x+32 column)
-  const int h = threadIdx.x;
+  const int tx = gtid % kTX, ty = gtid / kTX;  // ty in [0, kTB)
+  // halo role: the rows below and above the tile, the columns on both sides
+  const int h = gtid;
   int hx = -1, hy = -1;
   if (h < kTX) { hx = h + 1; hy = 0; }
   else if (h < 2 * kTX) { hx = h - kTX + 1; hy = kTY + 1; }
   else if (h < 2 * kTX + kTY) { hx = 0; hy = h - 2 * kTX + 1; }
   else if (h < 2 * kTX + 2 * kTY) { hx = kTX + 1; hy = h - 2 * kTX - kTY + 1; }
   int it = 0;
-  bool pending = false;
+  // x takes the directions of two iterations at a time, in odd iterations (the
+  // older one is read from the buffer that the new direction then replaces)
+  int pending = 0;  // directions not yet in x: pold's, and before it pnew's
   while (it + 1 <= maxiter) {
     it++;
     acc = 0.0;
     const double *r = V.r;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const bool upd = pending == 2;
+    for (int tile = blockIdx.x + grp * gridDim.x; tile < ntiles; tile += kCgG * gridDim.x) {
       const int tz = tile / (ntx * nty), rem = tile % (ntx * nty);
       const int i0 = 1 + (rem % ntx) * kTX, j0 = 1 + (rem / ntx) * kTY, k0 = 1 + tz * TZ;
       const int kend = min(k0 + TZ - 1, cz);
-      const int i = i0 + tx, ja = j0 + ty, jb = ja + 8;
+      const int i = i0 + tx, ja = j0 + ty, jb = ja + kTB;
       const bool inA = i <= cx && ja <= cy, inB = i <= cx && jb <= cy;
       const bool padA = i <= cx + 1 && ja <= cy + 1, padB = i <= cx + 1 && jb <= cy + 1;
       const int hi = i0 - 1 + hx, hj = j0 - 1 + hy;
       const bool hin = hx >= 0 && hi <= cx + 1 && hj <= cy + 1;
+      // the loads of a plane step: p_old and r of plane kk (and of the halo), and
+      // the coefficients and x of plane kk - 1; issued a step ahead
+      struct Step {
+        double nA, nB, rA, rB, hp, hr, axA, ayA, azA, xA, p2A, axB, ayB, azB, xB, p2B;
+      };
+      auto load = [&](int kk, Step &L) {
+        const int qA = i + PX * ja + PXY * kk, qB = qA + kTB * PX, cA = qA - PXY, cB = qB - PXY;
+        L = Step{};
+        if (padA) { L.nA = ld(pold + qA); if (it > 1) L.rA = ld(r + qA); }
+        if (padB) { L.nB = ld(pold + qB); if (it > 1) L.rB = ld(r + qB); }
+        if (hin) {
+          const int qh = hi + PX * hj + PXY * kk;
+          L.hp = ld(pold + qh);
+          if (it > 1) L.hr = ld(r + qh);
+        }
+        if (kk > k0) {
+          if (inA) { L.axA = V.acx[cA]; L.ayA = V.acy[cA]; L.azA = V.acz[cA]; if (upd) { L.xA = ld(V.x + cA); L.p2A = ld(pnew + cA); } }
+          if (inB) { L.axB = V.acx[cB]; L.ayB = V.acy[cB]; L.azB = V.acz[cB]; if (upd) { L.xB = ld(V.x + cB); L.p2B = ld(pnew + cB); } }
+        }
+      };
       double poA = 0.0, poB = 0.0;  // p_old of the plane being computed (kk - 1)
       double nA = 0.0, nB = 0.0;    // p_old of plane kk
+      Step nx;
+      load(k0 - 1, nx);
       for (int kk = k0 - 1; kk <= kend + 1; ++kk) {
         const int slot = (kk - k0 + 1) & 3;
         const bool comp = kk >= k0 + 1;
-        // issue every load of this plane step before using any of them
-        const int qA = i + PX * ja + PXY * kk, qB = qA + 8 * PX;
-        double rA = 0.0, rB = 0.0, hr = 0.0, hp = 0.0;
+        const Step cu = nx;
+        if (kk <= kend) load(kk + 1, nx);
         poA = nA; poB = nB;
-        nA = 0.0; nB = 0.0;
-        if (padA) { nA = ld(pold + qA); if (it > 1) rA = ld(r + qA); }
-        if (padB) { nB = ld(pold + qB); if (it > 1) rB = ld(r + qB); }
-        if (hin) {
-          const int qh = hi + PX * hj + PXY * kk;
-          hp = ld(pold + qh);
-          if (it > 1) hr = ld(r + qh);
-        }
-        const int cA = qA - PXY, cB = qB - PXY;
-        double axA = 0, ayA = 0, azA = 0, xA = 0, axB = 0, ayB = 0, azB = 0, xB = 0;
-        if (comp && inA) { axA = V.acx[cA]; ayA = V.acy[cA]; azA = V.acz[cA]; if (it > 1) xA = ld(V.x + cA); }
-        if (comp && inB) { axB = V.acx[cB]; ayB = V.acy[cB]; azB = V.acz[cB]; if (it > 1) xB = ld(V.x + cB); }
+        nA = cu.nA; nB = cu.nB;
+        const double rA = cu.rA, rB = cu.rB, hr = cu.hr, hp = cu.hp;
+        const int cA = i + PX * ja + PXY * (kk - 1), cB = cA + kTB * PX;
+        const double axA = cu.axA, ayA = cu.ayA, azA = cu.azA, xA = cu.xA, p2A = cu.p2A;
+        const double axB = cu.axB, ayB = cu.ayB, azB = cu.azB, xB = cu.xB, p2B = cu.p2B;
         pl[slot][ty + 1][tx + 1] = it == 1 ? nA : rA + beta * nA;
-        pl[slot][ty + 9][tx + 1] = it == 1 ? nB : rB + beta * nB;
+        pl[slot][ty + kTB + 1][tx + 1] = it == 1 ? nB : rB + beta * nB;
         if (hx >= 0) pl[slot][hy][hx] = it == 1 ? hp : hr + beta * hp;
-        __syncthreads();
+        group_sync();
         if (comp) {
           const int sc = (slot + 3) & 3, sb = (slot + 2) & 3;
           if (inA) {
@@ -1341,28 +1373,29 @@ __device__ void cg_core(const CgView &V, double bb, double tol, int maxiter, dou
             const double d = axA + axA + ayA + ayA + azA + azA;
             const double sv = d * c0 - azA * pl[sb][y][tx + 1] - ayA * pl[sc][y - 1][tx + 1] - axA * pl[sc][y][tx] -
                               axA * pl[sc][y][tx + 2] - ayA * pl[sc][y + 1][tx + 1] - azA * pl[slot][y][tx + 1];
-            if (it > 1) V.x[cA] = xA + alpha_prev * poA;
+            if (upd) V.x[cA] = (xA + alpha_prev2 * p2A) + alpha_prev * poA;
             pnew[cA] = c0;
             V.s[cA] = sv;
             acc += sv * c0;
           }
           if (inB) {
-            const int y = ty + 9;
+            const int y = ty + kTB + 1;
             const double c0 = pl[sc][y][tx + 1];
             const double d = axB + axB + ayB + ayB + azB + azB;
             const double sv = d * c0 - azB * pl[sb][y][tx + 1] - ayB * pl[sc][y - 1][tx + 1] - axB * pl[sc][y][tx] -
                               axB * pl[sc][y][tx + 2] - ayB * pl[sc][y + 1][tx + 1] - azB * pl[slot][y][tx + 1];
-            if (it > 1) V.x[cB] = xB + alpha_prev * poB;
+            if (upd) V.x[cB] = (xB + alpha_prev2 * p2B) + alpha_prev * poB;
             pnew[cB] = c0;
             V.s[cB] = sv;
             acc += sv * c0;
           }
         }
       }
-      __syncthreads();  // the next tile reuses the slots
+      group_sync();  // the next tile reuses the slots
     }
+    if (upd) pending = 0;
     const double sdotp = grid_sum(acc, partials, buf, sh, grid);
-    if (sdotp == 0.0) { pending = false; break; }
+    if (sdotp == 0.0) break;
     const double alpha = gamma / sdotp, gamma_old = gamma;
     acc = 0.0;
     {
@@ -1386,18 +1419,22 @@ __device__ void cg_core(const CgView &V, double bb, double tol, int maxiter, dou
     }
     gamma = grid_sum(acc, partials, buf, sh, grid);
     iprod = gamma;
+    alpha_prev2 = alpha_prev;
     alpha_prev = alpha;
-    pending = true;
+    ++pending;
     double *t = pold; pold = pnew; pnew = t;
     if (iprod / bb < eps) break;
     beta = gamma / gamma_old;
   }
-  if (pending)
+  if (pending == 1)
     for (long long e = tid; e < npad; e += T) V.x[e] = ld(V.x + e) + alpha_prev * ld(pold + e);
+  else if (pending == 2)
+    for (long long e = tid; e < npad; e += T)
+      V.x[e] = (ld(V.x + e) + alpha_prev2 * ld(pnew + e)) + alpha_prev * ld(pold + e);
   if (tid == 0) { *out_iters = it; *out_relres = sqrt(iprod / bb); }
 }
 
-__global__ void __launch_bounds__(kBlock) k_pcorr(FluidDev F, Prm P, double *partials, DevStats *st, int assemble,
+__global__ void __launch_bounds__(kCgT, 1) k_pcorr(FluidDev F, Prm P, double *partials, DevStats *st, int assemble,
                                                   int TZ) {
   cg::grid_group grid = cg::this_grid();
   __shared__ double sh[33];
@@ -1441,7 +1478,7 @@ __global__ void __launch_bounds__(kBlock) k_pcorr(FluidDev F, Prm P, double *par
 
 // Standalone HYPRE-rule CG on caller-provided padded arrays: r = p_a = b,
 // x = 0, then cg_core (hs_pcg_solve).
-__global__ void __launch_bounds__(kBlock) k_pcg(CgView V, const double *b, double tol, int maxiter, double *partials,
+__global__ void __launch_bounds__(kCgT, 1) k_pcg(CgView V, const double *b, double tol, int maxiter, double *partials,
                                                 int TZ, int *out_iters, double *out_relres) {
   cg::grid_group grid = cg::this_grid();
   __shared__ double sh[33];
@@ -1965,19 +2002,27 @@ int coop_blocks(K kernel, int nsm, int want) {
   return std::max(1, std::min(cap, want));
 }
 
-// z-depth of the CG tiles: balance tiles over the resident blocks and keep
-// the two halo planes a small share of each tile
-int choose_tz(long cx, long cy, long cz, int grid) {
-  long ntxy = ((cx + kTX - 1) / kTX) * ((cy + kTY - 1) / kTY);
-  double best = -1;
-  int tz_best = 16;
-  for (int tz = 4; tz <= 64; ++tz) {
-    long nt = ntxy * ((cz + tz - 1) / tz);
-    long rounds = (nt + grid - 1) / grid;
-    double eff = (double)cz / ((double)rounds * grid / ntxy * tz) * (double)tz / (tz + 2);
-    if (eff > best) { best = eff; tz_best = tz; }
+// z-depth of the CG tiles for `groups` thread groups: the fewest rounds of
+// (planes + the two halo planes)
+int choose_tz(long cx, long cy, long cz, int groups) {
+  const long ntxy = ((cx + kTX - 1) / kTX) * ((cy + kTY - 1) / kTY);
+  long best = -1;
+  int tz_best = 1;
+  for (int tz = 1; tz <= 64; ++tz) {
+    const long nt = ntxy * ((cz + tz - 1) / tz), cost = (nt + groups - 1) / groups * (tz + 2);
+    if (best < 0 || cost < best) { best = cost; tz_best = tz; }
   }
   return tz_best;
+}
+
+// blocks of a CG kernel (kCgT threads, kCgSmem bytes)
+template <class K>
+int cg_blocks(K kernel, int nsm, int want) {
+  int per = 0;
+  HS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmem));
+  HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kCgT, kCgSmem));
+  if (per < 1) throw std::runtime_error("cooperative kernel cannot be resident");
+  return std::max(1, std::min(nsm, want));
 }
 
 template <class K, class... A>
@@ -2195,8 +2240,8 @@ Engine::Engine(const Case &c, const hs_params &p, int device) : case_(c), prm_(p
     D.gs_prog = D.alloc<int>(tmax);
     D.gs_slots = D.alloc<double>((size_t)kTileW * wmax);
   }
-  D.g_pcorr = coop_blocks(k_pcorr, D.nsm, 1 << 30);
-  D.tz = choose_tz(M.cx, M.cy, M.cz, D.g_pcorr);
+  D.g_pcorr = cg_blocks(k_pcorr, D.nsm, 1 << 30);
+  D.tz = choose_tz(M.cx, M.cy, M.cz, D.g_pcorr * kCgG);
   D.snap = D.alloc<double>(std::max({M.nu(), M.nv(), M.nw(), M.npad(), 2 * (long)F.hs}));
   D.ssnap = D.alloc<double>(std::max<long long>(D.ntt, 1));
   D.spred = D.alloc<int>(std::max(D.nreg, 1));
@@ -2311,7 +2356,7 @@ void Engine::step(int nsteps) {
       coop_launch(k_mgcg, D.g_mgcg, kBlock, 0, s, D.F, D.P, D.mg, D.partials, D.stats);
     } else {
       Mark m(D, 3);
-      coop_launch(k_pcorr, D.g_pcorr, kBlock, 0, s, D.F, D.P, D.partials, D.stats, assemble, D.tz);
+      coop_launch(k_pcorr, D.g_pcorr, kCgT, kCgSmem, s, D.F, D.P, D.partials, D.stats, assemble, D.tz);
     }
     D.have_matrix = true;
     {
@@ -2547,8 +2592,8 @@ PcgWork *pcg_create(int nx, int ny, int nz, int device) {
   HS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
   std::unique_ptr<PcgWork> w(new PcgWork());
   w->device = device; w->cx = nx; w->cy = ny; w->cz = nz;
-  w->grid = coop_blocks(k_pcg, nsm, 1 << 30);
-  w->tz = choose_tz(nx, ny, nz, w->grid);
+  w->grid = cg_blocks(k_pcg, nsm, 1 << 30);
+  w->tz = choose_tz(nx, ny, nz, w->grid * kCgG);
   auto get = [](void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) throw std::runtime_error(std::string("CUDA alloc: ") + cudaGetErrorString(e));
@@ -2580,7 +2625,7 @@ void pcg_solve(PcgWork *w, const double *acx, const double *acy, const double *a
   HS_CUDA(cudaSetDevice(w->device));
   cudaStream_t st = (cudaStream_t)stream;
   CgView V{w->cx, w->cy, w->cz, acx, acy, acz, x, w->r, w->pa, w->pb, w->s};
-  coop_launch(k_pcg, w->grid, kBlock, 0, st, V, b, tol, maxiter, w->partials, w->tz, w->iters, w->relres);
+  coop_launch(k_pcg, w->grid, kCgT, kCgSmem, st, V, b, tol, maxiter, w->partials, w->tz, w->iters, w->relres);
   int it = 0;
   double rr = 0;
   HS_CUDA(cudaMemcpyAsync(&it, w->iters, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -2631,7 +2676,7 @@ NoAllocSetup noalloc_setup(int device) {
     void *ptr = nullptr;
     HS_CUDA(cudaGetSymbolAddress(&ptr, g_noalloc_scratch));
     HS_CUDA(cudaDeviceGetAttribute(&S.nsm, cudaDevAttrMultiProcessorCount, device));
-    S.grid = coop_blocks(k_pcg, S.nsm, kNoAllocMaxBlocks);
+    S.grid = cg_blocks(k_pcg, S.nsm, kNoAllocMaxBlocks);
     S.base = (double *)ptr;
   }
   return S;
@@ -2663,7 +2708,7 @@ void pcg_solve_noalloc(int nx, int ny, int nz, const double *acx, const double *
   // k_pcg writes every scratch word it later reads (r, p, s over the padded
   // grid, each partial before its reduction, both results), so the previous
   // call's contents never leak into this one
-  coop_launch(k_pcg, S.grid, kBlock, 0, st, V, b, tol, maxiter, partials, choose_tz(nx, ny, nz, S.grid), out_it, out_rel);
+  coop_launch(k_pcg, S.grid, kCgT, kCgSmem, st, V, b, tol, maxiter, partials, choose_tz(nx, ny, nz, S.grid * kCgG), out_it, out_rel);
   int it = 0;
   double rr = 0;
   HS_CUDA(cudaMemcpyAsync(&it, out_it, sizeof(int), cudaMemcpyDeviceToHost, st));
