@@ -1208,6 +1208,7 @@ struct ChannelState {
   CgVec<double> Vd{};
   CgVec<float> Vf{};
   double *scratch = nullptr;  // FP64 staging of field copies (padded cells)
+  double *keep_T = nullptr;   // the outer loop's T during an adjoint (from the first one on)
   mg::Hier<double> Gd{};
   mg::Hier<float> Gf{};
   int mom_blocks = 0, pcg_grid = 0;
@@ -1896,8 +1897,8 @@ void ch_adjoint(ChannelState *S, double tol, int maxiter, double *J, double *dJd
   CH_CUDA(cudaSetDevice(S->device));
   // the relaxed outer-loop temperature is kept; the adjoint works on a full solve
   const size_t np = (size_t)(S->N0 + 2) * (S->N1 + 2) * (S->N2 + 2);
-  double *keep = nullptr;
-  CH_CUDA(cudaMalloc(&keep, np * 8));
+  if (!S->keep_T) S->keep_T = S->alloc<double>(np);
+  double *keep = S->keep_T;
   CH_CUDA(cudaMemcpyAsync(keep, cht_T_device(S->cht), np * 8, cudaMemcpyDeviceToDevice, S->stream));
   cudaEvent_t e0, e1, e2;
   CH_CUDA(cudaEventCreate(&e0)); CH_CUDA(cudaEventCreate(&e1)); CH_CUDA(cudaEventCreate(&e2));
@@ -1918,7 +1919,6 @@ void ch_adjoint(ChannelState *S, double tol, int maxiter, double *J, double *dJd
   cudaEventDestroy(e0); cudaEventDestroy(e1); cudaEventDestroy(e2);
   CH_CUDA(cudaMemcpyAsync(cht_T_device(S->cht), keep, np * 8, cudaMemcpyDeviceToDevice, S->stream));
   CH_CUDA(cudaStreamSynchronize(S->stream));
-  cudaFree(keep);
 }
 
 }  // namespace hs

@@ -370,6 +370,16 @@ __global__ void k_cht_grad(ChtDev H, const double *T, const double *lam, double 
   }
 }
 
+// dJ/dk per region: block r sums its cells' shares (list: the regions' cells, in
+// cell order from first[r] on) in a fixed order
+__global__ void k_cht_dk(const int *first, const int *list, const double *dk_cell, double *dk) {
+  __shared__ double sh[32];
+  double a = 0.0;
+  for (int e = first[blockIdx.x] + threadIdx.x; e < first[blockIdx.x + 1]; e += blockDim.x) a += dk_cell[list[e]];
+  a = blk_sum(a, sh);
+  if (threadIdx.x == 0) dk[blockIdx.x] = a;
+}
+
 // face velocities of the global grid from the fluid box's u*, v*, w*; faces
 // outside the fluid box or touching a solid cell carry no flow
 __global__ void k_cht_velocities(ChtVelSrc S, double *ug, double *vg, double *wg) {
@@ -454,6 +464,8 @@ struct ChtState {
   uint8_t *solid = nullptr, *ctype_dev = nullptr;
   int *it = nullptr;
   std::vector<int> region;      // per global cell (-1 fluid)
+  int *reg_first = nullptr, *reg_list = nullptr;  // the regions' cells (k_cht_dk)
+  double *dk = nullptr;                           // dJ/dk per region
   std::vector<uint8_t> ctype;
   double J = 0;
   bool have_T = false;
@@ -543,6 +555,24 @@ ChtState *cht_create(const ChtSetup &S) {
   for (double **v : vec) *v = C->alloc<double>(np);
   C->T = C->alloc<double>(np); C->lam = C->alloc<double>(np); C->g = C->alloc<double>(np);
   C->dJdq = C->alloc<double>(n); C->dkc = C->alloc<double>(n);
+  {
+    // the solid cells region by region, each in cell order
+    std::vector<int> first(C->nreg + 1, 0), list;
+    auto mine = [&](size_t c) { return C->ctype[c] && C->region[c] >= 0 && C->region[c] < C->nreg; };
+    for (size_t c = 0; c < n; ++c)
+      if (mine(c)) ++first[C->region[c] + 1];
+    for (int r = 0; r < C->nreg; ++r) first[r + 1] += first[r];
+    list.resize(std::max(first[C->nreg], 1));
+    std::vector<int> at(first.begin(), first.end() - 1);
+    for (size_t c = 0; c < n; ++c)
+      if (mine(c)) list[at[C->region[c]]++] = (int)c;
+    C->reg_first = C->alloc<int>(first.size());
+    C->reg_list = C->alloc<int>(list.size());
+    C->dk = C->alloc<double>(C->nreg);
+    HC_CUDA(cudaMemcpyAsync(C->reg_first, first.data(), first.size() * 4, cudaMemcpyHostToDevice, C->stream));
+    HC_CUDA(cudaMemcpyAsync(C->reg_list, list.data(), list.size() * 4, cudaMemcpyHostToDevice, C->stream));
+    HC_CUDA(cudaStreamSynchronize(C->stream));  // the vectors go out of scope
+  }
   C->precond = S.precond;
   if (S.precond == 1) setup_levels(*C, C->Gf);
   if (S.precond == 2) setup_levels(*C, C->Gd);
@@ -672,7 +702,7 @@ void unpad(const ChtDev &H, const double *dev, double *host, cudaStream_t s) {
         host[i + (size_t)H.Nx * (j + (size_t)H.Ny * k)] = tmp[(i + 1) + (H.Nx + 2) * ((j + 1) + (size_t)(H.Ny + 2) * (k + 1))];
 }
 
-double objective(ChtState *C, bool grad) {
+double objective(ChtState *C) {
   const ChtDev &H = C->H;
   const int nb = gfor((long long)H.Nx * H.Ny * H.Nz);
   k_cht_objective<<<nb, kB, 0, C->stream>>>(H, C->T, C->g, C->partials);
@@ -681,9 +711,7 @@ double objective(ChtState *C, bool grad) {
   HC_CUDA(cudaStreamSynchronize(C->stream));
   double s = 0;
   for (double v : part) s += v;
-  const double J = std::pow(s, 1.0 / 8.0);
-  if (grad) k_cht_djdt<<<nb, kB, 0, C->stream>>>(H, C->T, std::pow(J, -7.0), C->g);
-  return J;
+  return std::pow(s, 1.0 / 8.0);
 }
 }  // namespace
 
@@ -700,7 +728,7 @@ void cht_forward(ChtState *C, double *T_host, double *J, int *iters, double *rel
   HC_CUDA(cudaMemcpyAsync(&it, C->it, 4, cudaMemcpyDeviceToHost, C->stream));
   HC_CUDA(cudaMemcpyAsync(&rr, C->res, 8, cudaMemcpyDeviceToHost, C->stream));
   HC_CUDA(cudaStreamSynchronize(C->stream));
-  C->J = objective(C, false);
+  C->J = objective(C);
   C->have_T = true;
   if (T_host) unpad(H, C->T, T_host, C->stream);
   if (J) *J = C->J;
@@ -714,26 +742,23 @@ void cht_adjoint(ChtState *C, double *dJdq_host, double *dJdk_host, int *iters, 
   const ChtDev &H = C->H;
   const size_t np = (size_t)(H.Nx + 2) * (H.Ny + 2) * (H.Nz + 2);
   const long long n = (long long)H.Nx * H.Ny * H.Nz;
-  objective(C, true);
+  // dJ/dT at the forward solve's T and J
+  k_cht_djdt<<<gfor(n), kB, 0, C->stream>>>(H, C->T, std::pow(C->J, -7.0), C->g);
   HC_CUDA(cudaMemsetAsync(C->V.x, 0, np * 8, C->stream));
   solve(C, C->g, 1, C->tol, C->maxiter, 0, nullptr);
   HC_CUDA(cudaMemcpyAsync(C->lam, C->V.x, np * 8, cudaMemcpyDeviceToDevice, C->stream));
   k_cht_grad<<<gfor(n), kB, 0, C->stream>>>(H, C->T, C->lam, C->Tb, C->dJdq, C->dkc);
   if (device_done) HC_CUDA(cudaEventRecord((cudaEvent_t)device_done, C->stream));
-  std::vector<double> dq(n), dk(n);
+  if (C->nreg > 0) k_cht_dk<<<C->nreg, kB, 0, C->stream>>>(C->reg_first, C->reg_list, C->dkc, C->dk);
+  HC_CUDA(cudaGetLastError());
   int it = 0;
   double rr = 0;
-  HC_CUDA(cudaMemcpyAsync(dq.data(), C->dJdq, n * 8, cudaMemcpyDeviceToHost, C->stream));
-  HC_CUDA(cudaMemcpyAsync(dk.data(), C->dkc, n * 8, cudaMemcpyDeviceToHost, C->stream));
   HC_CUDA(cudaMemcpyAsync(&it, C->it, 4, cudaMemcpyDeviceToHost, C->stream));
   HC_CUDA(cudaMemcpyAsync(&rr, C->res, 8, cudaMemcpyDeviceToHost, C->stream));
+  if (dJdk_host && C->nreg > 0)
+    HC_CUDA(cudaMemcpyAsync(dJdk_host, C->dk, (size_t)C->nreg * 8, cudaMemcpyDeviceToHost, C->stream));
+  if (dJdq_host) HC_CUDA(cudaMemcpyAsync(dJdq_host, C->dJdq, n * 8, cudaMemcpyDeviceToHost, C->stream));
   HC_CUDA(cudaStreamSynchronize(C->stream));
-  if (dJdq_host) std::copy(dq.begin(), dq.end(), dJdq_host);
-  if (dJdk_host) {
-    for (int r = 0; r < C->nreg; ++r) dJdk_host[r] = 0.0;
-    for (long long c = 0; c < n; ++c)
-      if (C->ctype[c]) dJdk_host[C->region[c]] += dk[c];
-  }
   if (iters) *iters = it;
   if (relres) *relres = rr;
 }
