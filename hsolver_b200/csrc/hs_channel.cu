@@ -694,7 +694,7 @@ __device__ double grid_sum(double v, double *partials, int &buf, double *sh, cg:
   grid.sync();
   double a = 0.0;
   if (threadIdx.x < 32) {
-    for (int q = threadIdx.x; q < (int)gridDim.x; q += 32) a += __ldcg(pp + q);
+    a = mg::lane_sum(pp, (int)gridDim.x, 1);
     for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (threadIdx.x == 0) sh[32] = a;
   }

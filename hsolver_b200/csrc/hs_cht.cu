@@ -92,8 +92,7 @@ __device__ void grid_sums(double (&v)[M], double *partials, int &buf, double *sh
   if (threadIdx.x < 32) {
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-      double a = 0.0;
-      for (int q = threadIdx.x; q < (int)gridDim.x; q += 32) a += __ldcg(pp + (size_t)q * M + m);
+      double a = mg::lane_sum(pp + m, (int)gridDim.x, M);
       for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
       if (threadIdx.x == 0) sh[40 + m] = a;
     }

@@ -154,8 +154,16 @@ __device__ double grid_sum(double v, double *partials, int &buf, double *sh, cg:
   if (threadIdx.x == 0) pp[blockIdx.x] = b;
   grid.sync();
   if (threadIdx.x < 32) {
+    // eight loads in flight (one after another: five trips to L2 for 148 blocks)
     double a = 0.0;
-    for (int q = threadIdx.x; q < (int)gridDim.x; q += 32) a += __ldcg(pp + q);
+    for (int q0 = threadIdx.x; q0 < (int)gridDim.x; q0 += 256) {
+      double w[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) w[u] = q0 + 32 * u < (int)gridDim.x ? __ldcg(pp + q0 + 32 * u) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (q0 + 32 * u < (int)gridDim.x) a += w[u];
+    }
     for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (threadIdx.x == 0) sh[32] = a;
   }

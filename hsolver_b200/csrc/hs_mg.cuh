@@ -99,6 +99,22 @@ struct Walk {
   __host__ __device__ __forceinline__ int flat() const { return m + mx * (j + ny * k); }
 };
 
+// This lane's part of a sum over n values at a stride (values lane, lane + 32,
+// ... in that order), eight loads in flight: one after another they made the
+// second half of every grid-wide sum five trips to L2
+__device__ __forceinline__ double lane_sum(const double *p, int n, int stride) {
+  double a = 0.0;
+  for (int q0 = threadIdx.x & 31; q0 < n; q0 += 256) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = q0 + 32 * u < n ? __ldcg(p + (size_t)(q0 + 32 * u) * stride) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (q0 + 32 * u < n) a += v[u];
+  }
+  return a;
+}
+
 // values in each padded array of level L (row pitch px)
 template <class M>
 __host__ __device__ __forceinline__ long long padded(const Level<M> &L) { return (long long)L.px * (L.ny + 2) * (L.nz + 2); }
