@@ -751,32 +751,27 @@ __device__ void mg_fine_and_rhs(const CgVec<M> &V, const mg::Level<M> &L0, doubl
   }
 }
 
-// The CG's two passes by runs of W consecutive padded cells of an interior
-// row per thread step (16 bytes: two FP64 or four FP32 values; aligned: the
-// row pitch is a multiple of four values): a fraction of the load and store
-// instructions of per-cell passes, which bound them rather than DRAM.  Lanes
-// outside the interior (the ghost cells and the row's padding) compute from
-// in-bounds loads and store the zeros those cells hold.  Every interior
-// cell's arithmetic is the per-cell pass's, term for term; only the order of
-// this thread's dot-product terms differs.  Per cell the mixed p' solve took
-// 3.39 ms per outer step at 256x128x128 against 3.11 by runs.
+// The mixed form's two CG passes by runs of four consecutive padded cells of
+// an interior row per thread step (aligned: the row pitch is a multiple of
+// four values), with 16-byte loads and stores: a quarter of the load and
+// store instructions of the per-cell passes, whose FP32 form was bound by
+// them rather than by DRAM bytes.  Lanes outside the interior (the ghost
+// cells and the row's padding) compute from in-bounds loads and store the
+// zeros those cells hold.  Every interior cell's arithmetic is the per-cell
+// pass's, term for term; only the order of this thread's dot-product terms
+// differs.  Mixed p' solve per outer step at 256x128x128: 3.39 ms per cell,
+// 3.11 ms by runs.  (FP64 by runs of two: 95 against 132 us per iteration for
+// the two passes, but another order of the dot products, and on stretched
+// grids, where a solve takes 40-50 iterations, that moves the fields by 1e-7:
+// the FP64 passes stay per cell.)
 template <int W>
 __device__ __forceinline__ void ldv(float (&v)[W], const float *p, bool cg_) {
   const float4 t = cg_ ? __ldcg(reinterpret_cast<const float4 *>(p)) : *reinterpret_cast<const float4 *>(p);
   v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
 }
 template <int W>
-__device__ __forceinline__ void ldv(double (&v)[W], const double *p, bool cg_) {
-  const double2 t = cg_ ? __ldcg(reinterpret_cast<const double2 *>(p)) : *reinterpret_cast<const double2 *>(p);
-  v[0] = t.x; v[1] = t.y;
-}
-template <int W>
 __device__ __forceinline__ void stv(float *p, const float (&v)[W]) {
   *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-template <int W>
-__device__ __forceinline__ void stv(double *p, const double (&v)[W]) {
-  *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
 }
 // p = z + beta p_old (or z in the first iteration) at the run q0
 template <class M, int W>
@@ -955,14 +950,42 @@ __global__ void __launch_bounds__(PcgT<M>::v, 1)
   while (it < maxiter && !(rr / bb < eps)) {
     const bool first = it == 0;
     it++;
+    acc = 0.0;
     const M bm = (M)beta;
+    auto pval = [&](int qq) -> M {
+      const M z = precond ? __ldcg(L0.x + qq) : __ldcg(V.r + qq);
+      return first ? z : z + bm * __ldcg(po + qq);
+    };
     // p in storage precision; the product in FP64 (in FP32 its cancellation
     // error for smooth p would reach the near-null modes of the p' system)
-    acc = cg_ap_runs(V, (const M *)(precond ? L0.x : V.r), (const M *)po, pn, first, bm, tid, T);
+    if constexpr (is_mixed(M())) acc = cg_ap_runs(V, (const M *)(precond ? L0.x : V.r), (const M *)po, pn, first, bm, tid, T);
+    else for (mg::Walk w(N0, N1, V.N2, tid, T); w.ok(); w.next()) {
+      const int q = (w.m + 1) + PX * ((w.j + 1) + PY * (w.k + 1));
+      const M p0 = pval(q);
+      const double cw = V.acx[q], ce = V.acx[q + 1], cs = V.acy[q], cn = V.acy[q + PX], cb = V.acz[q], cf = V.acz[q + PXY];
+      const double d = cw + ce + cs + cn + cb + cf;
+      const double sv = d * (double)p0 - (cw * (double)pval(q - 1) + ce * (double)pval(q + 1) + cs * (double)pval(q - PX) +
+                                          cn * (double)pval(q + PX) + cb * (double)pval(q - PXY) + cf * (double)pval(q + PXY));
+      pn[q] = p0;
+      V.s[q] = (M)sv;
+      acc += (double)(M)sv * (double)p0;
+    }
     const double sp = grid_sum(acc, partials, buf, sh, grid);
     if (sp == 0.0) break;
     const double alpha = gamma / sp;
-    acc = cg_update_runs(V, L0, precond != 0, (const M *)pn, alpha, tid, T);
+    acc = 0.0;
+    if constexpr (is_mixed(M())) acc = cg_update_runs(V, L0, precond != 0, (const M *)pn, alpha, tid, T);
+    else for (mg::Walk w(N0, N1, V.N2, tid, T); w.ok(); w.next()) {
+      const int q = (w.m + 1) + PX * ((w.j + 1) + PY * (w.k + 1));
+      const bool seed = precond && !((w.m + w.j + w.k) & 1);  // the V-cycle's rhs is r itself
+      const double xv = (double)V.x[q], pv = (double)pn[q], r0 = (double)V.r[q], sv = (double)V.s[q];
+      const M d = seed ? L0.d[q] : M(0);
+      V.x[q] = (M)(xv + alpha * pv);
+      const M rv = (M)(r0 - alpha * sv);
+      V.r[q] = rv;
+      acc += (double)rv * (double)rv;
+      if (seed) L0.x[q] = d == M(0) ? M(0) : rv / d;
+    }
     rr = grid_sum(acc, partials, buf, sh, grid);
     if (rr / bb < eps || it >= maxiter) break;  // no V-cycle for an iteration that will not run
     const double gnew = precond ? rz() : rr;
