@@ -156,7 +156,8 @@ __global__ void __launch_bounds__(kB, 4) k_cht_assemble(ChtDev H, double Tb, mg:
         else if (last) { g[q + st] = (MT)G; f[q + st] = (MT)F; }
       }
     }
-    H.d[q] = diag; H.dinv[q] = 1.0 / diag;
+    H.d[q] = diag;
+    if (!L0.gx) H.dinv[q] = 1.0 / diag;  // the Jacobi preconditioner's
     H.aw[q] = a[0]; H.ae[q] = a[1]; H.as[q] = a[2]; H.an[q] = a[3]; H.ab[q] = a[4]; H.af[q] = a[5];
     H.b[q] = rhs;
   }
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(kBiT, 1) k_cht_bicgstab(ChtDev H, VecT<VT> V, 
       if (x0) V.x[q] = VT(0);
     }
     const double rv = bq - ax;
-    V.r[q] = (VT)rv; V.rh[q] = (VT)rv; V.p[q] = VT(0); V.v[q] = VT(0);
+    V.r[q] = (VT)rv; V.rh[q] = (VT)rv;
     red[0] += bq * bq;
     red[1] += rv * rv;
   }
@@ -235,10 +236,11 @@ __global__ void __launch_bounds__(kBiT, 1) k_cht_bicgstab(ChtDev H, VecT<VT> V, 
   while (it < maxiter && !(rr / bb < eps)) {
     it++;
     const double beta = (rho1 / rho) * (alpha / omega);
-    // each pass issues every load of a cell before its first store
+    // each pass issues every load of a cell before its first store; p and v start at 0
+    const bool first = it == 1;
     for (mg::Walk w(Nx, Ny, H.Nz, tid, T); w.ok(); w.next()) {
       const int q = (w.m + 1) + PX * ((w.j + 1) + (Ny + 2) * (w.k + 1));
-      const double r_ = (double)V.r[q], p_ = (double)V.p[q], v_ = (double)V.v[q];
+      const double r_ = (double)V.r[q], p_ = first ? 0.0 : (double)V.p[q], v_ = first ? 0.0 : (double)V.v[q];
       const mg::Seed<MT> sd = mgp ? mg::seed_at(Gm.lv[0], w.m, w.j, w.k, q, tr) : mg::Seed<MT>{};
       const double di = mgp ? 0.0 : H.dinv[q];
       const VT pv = (VT)(r_ + beta * (p_ - omega * v_));
