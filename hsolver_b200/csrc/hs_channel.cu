@@ -1252,9 +1252,11 @@ struct ChannelState {
   // statistics of the steps of one ch_step call, copied without waiting
   // (pinned), applied in order after one stream synchronisation per kRing steps
   struct StepRec {
-    double res[4], prel, trr[2];
+    double res[4], prel;
     int pit, tit;
+    double trr[2];
   };
+  StepRec *rec_dev = nullptr;  // the kernels' results of a step: one copy (five took ~15 us of a small step)
   static constexpr int kRing = 64;
   StepRec *ring = nullptr;
   cudaEvent_t ev[6] = {};
@@ -1572,11 +1574,8 @@ void step_once(ChannelState &S, ChDev<R> &H, int flags) {
 
 // the step's statistics into rec, on the stream (rec in pinned memory: the
 // copies do not wait; read rec after the stream has passed them)
-void enqueue_stats(ChannelState &S, ChannelState::StepRec &rec, int flags) {
-  CH_CUDA(cudaMemcpyAsync(rec.res, S.res, 32, cudaMemcpyDeviceToHost, S.stream));
-  CH_CUDA(cudaMemcpyAsync(&rec.pit, S.pcg_it, 4, cudaMemcpyDeviceToHost, S.stream));
-  CH_CUDA(cudaMemcpyAsync(&rec.prel, S.pcg_rel, 8, cudaMemcpyDeviceToHost, S.stream));
-  if (!(flags & 2)) cht_step_results_async(S.cht, &rec.tit, rec.trr);
+void enqueue_stats(ChannelState &S, ChannelState::StepRec &rec) {
+  CH_CUDA(cudaMemcpyAsync(&rec, S.rec_dev, sizeof rec, cudaMemcpyDeviceToHost, S.stream));
 }
 
 // the step's bookkeeping from its statistics: residuals, the normalisers
@@ -1605,7 +1604,7 @@ void apply_stats(ChannelState &S, const ChannelState::StepRec &rec, int flags) {
 
 void read_stats(ChannelState &S, int flags) {
   ChannelState::StepRec &rec = S.ring[0];
-  enqueue_stats(S, rec, flags);
+  enqueue_stats(S, rec);
   CH_CUDA(cudaStreamSynchronize(S.stream));
   if (S.prof) {
     for (int ph = 0; ph < 5; ++ph) {
@@ -1683,7 +1682,8 @@ ChannelState *ch_create(const Case &c, const ChParams &p, int device) {
       &per, S->mixed ? (const void *)k_ch_mom<float, 0> : (const void *)k_ch_mom<double, 0>, kT, 0));
   S->mom_blocks = std::min(blocks_for(nmax), std::max(1, per * nsm / 3));
   S->mom_part = S->alloc<double>((size_t)3 * S->mom_blocks);
-  S->res = S->alloc<double>(4);
+  S->rec_dev = S->alloc<ChannelState::StepRec>(1);
+  S->res = S->rec_dev->res;
   S->asm_blocks = blocks_for(nmax);
   S->cont_part = S->alloc<double>((size_t)S->asm_blocks);
   // the four-part correction: at least 148 x 8 chunks per part (fewer on a
@@ -1702,8 +1702,8 @@ ChannelState *ch_create(const Case &c, const ChParams &p, int device) {
   if (S->mixed) setup_zm(*S, S->Vf, S->Gf, S->TMf, nsm);
   else setup_zm(*S, S->Vd, S->Gd, S->TMd, nsm);
   S->pcg_part = S->alloc<double>((size_t)4 * std::max(S->pcg_grid, S->zm_grid) + 64);
-  S->pcg_it = S->alloc<int>(1);
-  S->pcg_rel = S->alloc<double>(1);
+  S->pcg_it = &S->rec_dev->pit;
+  S->pcg_rel = &S->rec_dev->prel;
   // energy: the conjugate-heat-transfer operator in channel mode, on this stream
   S->region.resize(n);
   for (size_t i = 0; i < n; ++i) S->region[i] = c.ctype[i] ? c.region[i] : -1;
@@ -1717,6 +1717,7 @@ ChannelState *ch_create(const Case &c, const ChParams &p, int device) {
   cs.step_fp32 = p.precision == 1;
   S->cht = cht_create(cs);
   CH_CUDA(cudaHostAlloc((void **)&S->ring, ChannelState::kRing * sizeof(ChannelState::StepRec), cudaHostAllocDefault));
+  cht_bind_results(S->cht, &S->rec_dev->tit, S->rec_dev->trr);
   cht_bind_velocities(S->cht, uarr(S.get(), 0), uarr(S.get(), 1), uarr(S.get(), 2));
   if (S->mixed) S->Hf.T = cht_T_device(S->cht);
   else S->Hd.T = cht_T_device(S->cht);
@@ -1778,7 +1779,7 @@ void ch_step(ChannelState *S, int n, int flags, ChStats *out) {
       for (int s = 0; s < b; ++s) {
         if (S->mixed) step_once(*S, S->Hf, flags);
         else step_once(*S, S->Hd, flags);
-        enqueue_stats(*S, S->ring[s], flags);
+        enqueue_stats(*S, S->ring[s]);
       }
       CH_CUDA(cudaStreamSynchronize(S->stream));
       for (int s = 0; s < b; ++s) apply_stats(*S, S->ring[s], flags);
