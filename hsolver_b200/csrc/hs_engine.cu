@@ -976,7 +976,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_gs_planes(FluidDev F, Prm P, doub
 // ---------------------------------------------------------------- solid energy
 // MobSolver::solve (mobs_solver.h:303-319) with solveTemperature
 // (mobs_solver.h:467-500) for every solid region at once, pipelined and
-// speculated like k_gs; each region keeps its own residual, stop test and
+// speculated like k_gs_planes; each region keeps its own residual, stop test and
 // sweep count.
 constexpr int kMaxRegions = 256;
 __global__ void __launch_bounds__(kBlock, 2) k_solid(const SolidReg *regs, int nreg, const int *blk_reg, double *tt_all,
