@@ -1419,8 +1419,8 @@ void setup_mg(ChannelState &S, mg::Hier<M> &G, const CgVec<M> &V, int nsm) {
     l.nx = nx; l.ny = ny; l.nz = nz; l.px = pitch4(nx + 2);
     const size_t np = (size_t)l.px * (ny + 2) * (nz + 2);
     l.x = S.alloc<M>(np);
-    // level 0's rhs is the CG's residual (the z-marching form keeps a buffer of its own there)
-    l.rhs = L == 0 && S.prm.p_level0 != 2 ? V.r : S.alloc<M>(np);
+    // level 0's rhs is the CG's residual (setup_zm gives the z-marching form a buffer of its own there)
+    l.rhs = L == 0 ? V.r : S.alloc<M>(np);
     if (L == 0) {  // the p' couplings themselves (written by the assembly, read-only in the solve)
       l.gx = const_cast<M *>(V.acx); l.gy = const_cast<M *>(V.acy); l.gz = const_cast<M *>(V.acz);
       l.d = S.alloc<M>(np);
@@ -1492,6 +1492,18 @@ void setup_zm(ChannelState &S, CgVec<M> &V, mg::Hier<M> &G, PcgMaps &TM, int nsm
   // p_level0: 0 the faster form on this pool (the grid-wide passes until the
   // z-marching ones beat them), 1 grid-wide, 2 z-marching
   if (!S.prm.p_precond || S.prm.p_level0 != 2 || G.L < 2 || G.ls < 1) return;
+  // the ring shares the launch's dynamic shared memory with block 0's staging
+  // of the small levels, which therefore holds their x and rhs only (the
+  // read-only arrays would not survive the ring between V-cycles)
+  mg::plan_stage(G, false);
+  const size_t smem = std::max<size_t>((size_t)zm::Box<M>::SMEM + 128, (size_t)G.stage);
+  CH_CUDA(cudaFuncSetAttribute((const void *)k_ch_pcg_zm<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per = 0;
+  CH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)k_ch_pcg_zm<M>, zm::kThreads, smem));
+  if (per < 1) return;
+  // the grid-wide passes take the residual itself as level 0's rhs, so the
+  // buffer of this form is made only where this form runs
+  G.lv[0].rhs = S.alloc<M>((size_t)mg::padded(G.lv[0]));
   const EncodeTiled enc = tensor_map_encoder();
   const int py = S.N1 + 2, pz = S.N2 + 2;
   auto fine = [&](const M *a) { return padded_map<M>(enc, a, S.PX, py, pz, zm::Box<M>::BX, zm::Box<M>::BY); };
@@ -1502,15 +1514,6 @@ void setup_zm(ChannelState &S, CgVec<M> &V, mg::Hier<M> &G, PcgMaps &TM, int nsm
   TM.s = fine(V.s);
   const mg::Level<M> &L1 = G.lv[1];
   TM.x1 = padded_map<M>(enc, L1.x, L1.px, L1.ny + 2, L1.nz + 2, zm::Box<M>::CBX, zm::Box<M>::CBY);
-  // the ring shares the launch's dynamic shared memory with block 0's staging
-  // of the small levels, which therefore holds their x and rhs only (the
-  // read-only arrays would not survive the ring between V-cycles)
-  mg::plan_stage(G, false);
-  const size_t smem = std::max<size_t>((size_t)zm::Box<M>::SMEM + 128, (size_t)G.stage);
-  CH_CUDA(cudaFuncSetAttribute((const void *)k_ch_pcg_zm<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per = 0;
-  CH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)k_ch_pcg_zm<M>, zm::kThreads, smem));
-  if (per < 1) return;
   S.zm_grid = per * nsm;
   S.zm_smem = smem;
   V.nch = zm::pick_chunks(((S.N0 + zm::kTX - 1) / zm::kTX) * ((S.N1 + zm::kTY - 1) / zm::kTY), S.N2, S.zm_grid);
