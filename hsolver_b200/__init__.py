@@ -75,6 +75,7 @@ def load(path=LIB_PATH):
     L.hs_init.argtypes = [vp]
     L.hs_step.argtypes = [vp, ctypes.c_int, ctypes.POINTER(Stats)]
     L.hs_sync.argtypes = [vp]
+    L.hs_set_wait_limit.argtypes = [vp, ctypes.c_int]
     L.hs_field_size.argtypes = [vp, ctypes.c_int, llp]
     L.hs_get_field.argtypes = [vp, ctypes.c_int, dp, ll]
     L.hs_set_field.argtypes = [vp, ctypes.c_int, dp, ll]
@@ -159,6 +160,10 @@ class Solver:
 
     def sync(self):
         self._check(self._L.hs_sync(self.h))
+
+    def set_wait_limit(self, polls):
+        """Polls after which a wait between the tiles of a sweep gives up (hs_set_wait_limit)."""
+        self._check(self._L.hs_set_wait_limit(self.h, polls))
 
     def field_size(self, name):
         n = ctypes.c_longlong()

@@ -163,6 +163,10 @@ int hs_sync(hs_ctx *ctx) {
   return guarded(ctx, [](hs::Engine &e) { e.sync(); return HS_OK; });
 }
 
+int hs_set_wait_limit(hs_ctx *ctx, int polls) {
+  return guarded(ctx, [&](hs::Engine &e) { e.set_wait_limit(polls); return HS_OK; });
+}
+
 int hs_stream(hs_ctx *ctx, void **stream) {
   if (!stream) return fail(ctx, HS_ERR_ARG, "null output pointer");
   return guarded(ctx, [&](hs::Engine &e) { *stream = e.stream_handle(); return HS_OK; });

@@ -365,7 +365,7 @@ constexpr int kGsT = 128;        // threads per block: four warps, spread over t
 // flight (256x128x128 energy: one sweep 0.5 against 1.6 ms, 100 sweeps 34
 // against 15).
 constexpr int kTileW = 4;
-constexpr int kGsSpin = 1 << 21; // polls before a wait gives up (about a second)
+constexpr int kGsSpin = 1 << 21; // polls before a wait gives up (about a second), unless set (hs_set_wait_limit)
 constexpr int kGsRing = 32, kGsPitch = 35;  // i values per staged row; its pitch (the lanes' rows and skew in distinct banks)
 
 // The staged arrays of an equation: its own field and the three others it
@@ -493,22 +493,24 @@ __device__ __forceinline__ double gs_update(const FluidDev &F, const Prm &P, int
 struct GsFlags {
   int *prog;       // one per tile
   int *give_up, *told;  // set by the first wait that runs out (device, host memory); no wait is taken after it
+  int limit;       // polls before a wait runs out (0: at once)
   bool dead;
-  // lanes 0..3 hold one tile index and the count it must have reached (idx < 0: none)
+  // lanes 0..3 hold one tile index and the count it must have reached (idx < 0: none).
+  // Whether the wait ends is decided by the warp as a whole: its lanes read
+  // give_up at different moments, and a lane that left the loop alone would
+  // leave the others waiting for it at the vote.
   __device__ __forceinline__ void wait(int idx, int need) {
-    if (!dead) {
-      int spins = 0;
-      while (true) {
-        int v = need;
-        if (idx >= 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(prog + idx) : "memory");
-        if (__all_sync(0xffffffffu, v >= need)) break;
-        ++spins;
-        if ((spins & 1023) == 0 && (spins >= kGsSpin || *(volatile int *)give_up)) {
-          dead = true;
+    for (int spins = 0; !dead; ++spins) {
+      if (spins == limit || (spins & 1023) == 1023) {
+        dead = __any_sync(0xffffffffu, spins == limit || *(volatile int *)give_up);
+        if (dead) {
+          if ((threadIdx.x & 31) == 0) *(volatile int *)give_up = *(volatile int *)told = 1;
           break;
         }
       }
-      if (dead && (threadIdx.x & 31) == 0) *(volatile int *)give_up = *(volatile int *)told = 1;
+      int v = need;
+      if (idx >= 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(prog + idx) : "memory");
+      if (__all_sync(0xffffffffu, v >= need)) break;
     }
     __syncwarp();
   }
@@ -690,9 +692,10 @@ __device__ double gs_tile(const FluidDev &F, const Prm &P, double *own, double *
 // One GS solve of equation EQ (0 u, 1 v, 2 w momentum; 3 fluid energy), as far
 // as its windows have at most kTileW sweeps; a larger one is left to
 // k_gs_planes.  prog: one counter per tile; slots: window residuals, one per
-// sweep and warp; told: set when a wait runs out (host memory: not for polling).
+// sweep and warp; told: set when a wait runs out (host memory: not for polling);
+// spin_limit: the polls after which one does.
 template <int EQ>
-__global__ void __launch_bounds__(kGsT, 1) k_gs_tiles(FluidDev F, Prm P, double *slots, int *prog, int *told, DevStats *st, double *snap) {
+__global__ void __launch_bounds__(kGsT, 1) k_gs_tiles(FluidDev F, Prm P, double *slots, int *prog, int *told, int spin_limit, DevStats *st, double *snap) {
   cg::grid_group grid = cg::this_grid();
   __shared__ double tot[kTileW];
   const int NI = EQ == 0 ? F.fx - 1 : F.cx, NJ = EQ == 1 ? F.fy - 1 : F.cy, NK = EQ == 2 ? F.fz - 1 : F.cz;
@@ -711,7 +714,7 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_tiles(FluidDev F, Prm P, double 
   const bool lid_row = (F.oy - 1 + F.fy - 1 == F.Ny);
   const int nJ = (NJ + kTJ - 1) / kTJ, nK = (NK + kTK - 1) / kTK, ntile = nJ * nK;
   const int nch = (NI + kTJ + kTK - 2 + kGsCh - 1) / kGsCh;
-  GsFlags fl{prog, &st->gave_up, told, false};
+  GsFlags fl{prog, &st->gave_up, told, spin_limit, false};
   const int pred = st->sweeps[EQ] > 0 ? st->sweeps[EQ] : 2;
   double residual = 1.0, gres = 1.0;
   int done = 0;
@@ -1946,6 +1949,7 @@ struct DeviceState {
   int *gs_prog = nullptr;      // the wavefront tiles' progress
   double *gs_slots = nullptr;  // window residuals per sweep and warp
   int *gave_up = nullptr;      // pinned: a wait between tiles ran out
+  int gs_spin = kGsSpin;       // polls after which one does
   // after the stream has been waited for
   void check_waits() const {
     if (*(volatile int *)gave_up)
@@ -2343,17 +2347,17 @@ void Engine::step(int nsteps) {
     // FluidSolver::solve (fluid_solver.h:1401-1633)
     {
       Mark m(D, 0);
-      coop_launch(k_gs_tiles<0>, D.g_tiles[0], kGsT, gs_smem<0>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.stats, D.snap);
+      coop_launch(k_gs_tiles<0>, D.g_tiles[0], kGsT, gs_smem<0>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.gs_spin, D.stats, D.snap);
       coop_launch(k_gs_planes<0>, D.g_gs[0], kBlock, 0, s, D.F, D.P, D.partials, D.stats, D.snap);
     }
     {
       Mark m(D, 1);
-      coop_launch(k_gs_tiles<1>, D.g_tiles[1], kGsT, gs_smem<1>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.stats, D.snap);
+      coop_launch(k_gs_tiles<1>, D.g_tiles[1], kGsT, gs_smem<1>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.gs_spin, D.stats, D.snap);
       coop_launch(k_gs_planes<1>, D.g_gs[1], kBlock, 0, s, D.F, D.P, D.partials, D.stats, D.snap);
     }
     {
       Mark m(D, 2);
-      coop_launch(k_gs_tiles<2>, D.g_tiles[2], kGsT, gs_smem<2>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.stats, D.snap);
+      coop_launch(k_gs_tiles<2>, D.g_tiles[2], kGsT, gs_smem<2>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.gs_spin, D.stats, D.snap);
       coop_launch(k_gs_planes<2>, D.g_gs[2], kBlock, 0, s, D.F, D.P, D.partials, D.stats, D.snap);
     }
     int assemble = (!D.have_matrix || !prm_.frozen_matrix) ? 1 : 0;
@@ -2374,7 +2378,7 @@ void Engine::step(int nsteps) {
     }
     {
       Mark m(D, 5);
-      coop_launch(k_gs_tiles<3>, D.g_tiles[3], kGsT, gs_smem<3>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.stats, D.snap);
+      coop_launch(k_gs_tiles<3>, D.g_tiles[3], kGsT, gs_smem<3>(), s, D.F, D.P, D.gs_slots, D.gs_prog, D.gave_up, D.gs_spin, D.stats, D.snap);
       coop_launch(k_gs_planes<3>, D.g_gs[3], kBlock, 0, s, D.F, D.P, D.partials, D.stats, D.snap);
     }
     // MobSolver::solve for every region
@@ -2505,6 +2509,11 @@ void Engine::sync() {
   HS_CUDA(cudaSetDevice(device_));
   HS_CUDA(cudaStreamSynchronize(d_->stream));
   d_->check_waits();
+}
+
+void Engine::set_wait_limit(int polls) {
+  if (polls < 0) throw std::invalid_argument("negative wait limit");
+  d_->gs_spin = polls;
 }
 
 void Engine::stats(hs_stats *out) {

@@ -25,6 +25,7 @@ class Engine {
   void init();
   void step(int n);
   void sync();
+  void set_wait_limit(int polls);
   void stats(hs_stats *out);
   void profile(bool on);
   int profile_read(double *ms, int nphase);

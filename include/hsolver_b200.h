@@ -102,6 +102,12 @@ int hs_step(hs_ctx *ctx, int n, hs_stats *stats);
 
 /* Wait for the context's stream. */
 int hs_sync(hs_ctx *ctx);
+/* The tiles of a Gauss-Seidel sweep wait for one another's progress on the
+ * GPU.  A wait that is not met within a number of polls (default 2^21, about
+ * a second; 0: at once) gives up: the sweep is abandoned, the step ends, and
+ * the next call that waits for the stream and reads (hs_sync, hs_step with
+ * stats, hs_get_field, hs_get_solid) returns HS_ERR_INTERNAL. */
+int hs_set_wait_limit(hs_ctx *ctx, int polls);
 /* The context's cudaStream_t (as void*), for callers that order their own
  * work after hs_step. */
 int hs_stream(hs_ctx *ctx, void **stream);

@@ -1,0 +1,57 @@
+"""A wait between the tiles of a wavefront sweep that runs out.  A limit of no
+polls makes every wait run out at its first call, whatever the other tiles
+have done: the kernels still return, and the calls that read report it."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HS_ERR_INTERNAL = -8
+BLOCKS = [(5, 20, 3, 9, 4, 8)]
+
+
+def _solver(dims=(33, 16, 12), blocks=BLOCKS, **prm):
+    import hsolver_b200
+    from hsolver_b200 import cases
+    s = hsolver_b200.Solver(cases.channel(*dims, blocks), hsolver_b200.default_params(pcg_maxiter=5, **prm))
+    s.init()
+    return s
+
+
+def _fails(call, *args, **kw):
+    import hsolver_b200
+    with pytest.raises(hsolver_b200.HsError) as e:
+        call(*args, **kw)
+    assert e.value.code == HS_ERR_INTERNAL and "ran out" in str(e.value)
+
+
+# one tile, a few, more than the resident warps
+@pytest.mark.parametrize("dims,blocks", [((7, 8, 5), [(3, 4, 3, 4, 2, 3)]), ((33, 16, 12), BLOCKS),
+                                         ((5, 203, 107), [(2, 4, 30, 60, 20, 40)])])
+@pytest.mark.parametrize("gs_max", [1, 3])
+def test_a_wait_that_runs_out_is_reported(dims, blocks, gs_max):
+    s = _solver(dims, blocks, gs_max=gs_max)
+    s.set_wait_limit(0)
+    s.step(2)
+    _fails(s.sync)
+    _fails(s.step, 1, stats=True)
+    _fails(s.field, "ux")
+    _fails(s.solid, 0)
+    s.close()
+
+
+def test_the_limit_leaves_results_alone():
+    a, b = _solver(), _solver()
+    b.set_wait_limit(1 << 20)
+    for s in (a, b):
+        s.step(3)
+    for f in ("u_star", "v_star", "w_star", "t_temp", "ux", "p", "t"):
+        assert np.array_equal(a.field(f), b.field(f)), f
+
+
+def test_negative_limit_is_refused():
+    import hsolver_b200
+    s = _solver()
+    with pytest.raises(hsolver_b200.HsError) as e:
+        s.set_wait_limit(-1)
+    assert e.value.code == -1
