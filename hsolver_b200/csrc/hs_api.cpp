@@ -492,22 +492,25 @@ int hs_cht_forward(hs_cht *h, double *T, double *J, int *iters, double *relres) 
     V.ctype = nullptr;
     hs::cht_set_velocities(h->st, V);
     hs::cht_forward(h->st, T, J, iters, relres);
+    e.check_waits();  // of the steps that left these velocities
     return HS_OK;
   });
 }
 
 int hs_cht_adjoint(hs_cht *h, double *dJdq, double *dJdk, int *iters, double *relres) {
   if (!h) return fail(nullptr, HS_ERR_ARG, "null handle");
-  return guarded(h->ctx, [&](hs::Engine &) {
+  return guarded(h->ctx, [&](hs::Engine &e) {
     hs::cht_adjoint(h->st, dJdq, dJdk, iters, relres);
+    e.check_waits();
     return HS_OK;
   });
 }
 
 int hs_cht_velocities(hs_cht *h, double *ug, double *vg, double *wg) {
   if (!h || !ug || !vg || !wg) return fail(nullptr, HS_ERR_ARG, "null argument");
-  return guarded(h->ctx, [&](hs::Engine &) {
+  return guarded(h->ctx, [&](hs::Engine &e) {
     hs::cht_get_velocities(h->st, ug, vg, wg);
+    e.check_waits();
     return HS_OK;
   });
 }

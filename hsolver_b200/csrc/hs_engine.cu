@@ -2430,6 +2430,7 @@ int Engine::profile_read(double *ms, int nphase) {
     D.ev_pool.push_back(u.second.second);
   }
   D.ev_used.clear();
+  D.check_waits();
   return count;
 }
 
@@ -2438,6 +2439,7 @@ void Engine::counters(long long *out8) {
   HS_CUDA(cudaMemcpyAsync(D.stats_host, D.stats, sizeof(DevStats), cudaMemcpyDeviceToHost, D.stream));
   HS_CUDA(cudaStreamSynchronize(D.stream));
   const DevStats &h = *D.stats_host;
+  D.check_waits();
   out8[0] = h.cum_sweeps[0]; out8[1] = h.cum_sweeps[1]; out8[2] = h.cum_sweeps[2]; out8[3] = h.cum_sweeps[3];
   out8[4] = h.cum_solid_cell_sweeps; out8[5] = h.cum_pcg_iters; out8[6] = h.cum_pcg_solves; out8[7] = steps_;
 }
@@ -2558,7 +2560,12 @@ long Engine::field_size(int f) const {
   return n;
 }
 
-double *Engine::field_device_ptr(int f, long *n) { return field_ptr(*d_, case_.fluid, f, n); }
+double *Engine::field_device_ptr(int f, long *n) {
+  d_->check_waits();
+  return field_ptr(*d_, case_.fluid, f, n);
+}
+
+void Engine::check_waits() const { d_->check_waits(); }
 
 void Engine::get_field(int f, double *host, long n) {
   HS_CUDA(cudaSetDevice(device_));

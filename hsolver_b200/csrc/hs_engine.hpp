@@ -26,6 +26,8 @@ class Engine {
   void step(int n);
   void sync();
   void set_wait_limit(int polls);
+  // throws once the stream has been waited for past a sweep that was abandoned
+  void check_waits() const;
   void stats(hs_stats *out);
   void profile(bool on);
   int profile_read(double *ms, int nphase);

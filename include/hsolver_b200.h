@@ -106,7 +106,9 @@ int hs_sync(hs_ctx *ctx);
  * GPU.  A wait that is not met within a number of polls (default 2^21, about
  * a second; 0: at once) gives up: the sweep is abandoned, the step ends, and
  * the next call that waits for the stream and reads (hs_sync, hs_step with
- * stats, hs_get_field, hs_get_solid) returns HS_ERR_INTERNAL. */
+ * stats, hs_get_field, hs_get_solid, hs_counters, hs_profile_read, hs_cht_*
+ * on the context's flow) returns HS_ERR_INTERNAL.  hs_field_device_ptr does
+ * not wait: who reads through it calls hs_sync after hs_step and before. */
 int hs_set_wait_limit(hs_ctx *ctx, int polls);
 /* The context's cudaStream_t (as void*), for callers that order their own
  * work after hs_step. */

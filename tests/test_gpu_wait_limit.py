@@ -40,6 +40,29 @@ def test_a_wait_that_runs_out_is_reported(dims, blocks, gs_max):
     s.close()
 
 
+def test_every_reader_reports_it():
+    """The calls that hand out the step's outcome without copying a field:
+    counters, phase times, device addresses and the energy solve on the
+    engine's velocities."""
+    from hsolver_b200.adjoint import ChtProblem
+    s = _solver()
+    s.profile(True)
+    prob = ChtProblem(s, k_fluid=1.0, maxiter=10)
+    try:
+        k, q = np.full(prob.nreg, 10.0), np.zeros(33 * 16 * 12)
+        prob.forward(k, q)
+        s.set_wait_limit(0)
+        s.step(1)
+        _fails(prob.velocities)
+        _fails(prob.gradient)
+        _fails(prob.forward, k, q)
+        _fails(s.counters)
+        _fails(s.profile_read)
+        _fails(s.device_ptr, "u_star")
+    finally:
+        prob.__del__()  # before its solver
+
+
 def test_the_limit_leaves_results_alone():
     a, b = _solver(), _solver()
     b.set_wait_limit(1 << 20)
