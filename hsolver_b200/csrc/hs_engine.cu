@@ -1950,10 +1950,13 @@ struct DeviceState {
   double *gs_slots = nullptr;  // window residuals per sweep and warp
   int *gave_up = nullptr;      // pinned: a wait between tiles ran out
   int gs_spin = kGsSpin;       // polls after which one does
+  bool told = false;           // and a caller has been told
   // after the stream has been waited for
-  void check_waits() const {
-    if (*(volatile int *)gave_up)
-      throw std::runtime_error("Gauss-Seidel sweep: a wait between tiles ran out (the sweep was abandoned)");
+  bool abandoned() const { return *(volatile int *)gave_up != 0; }
+  void check_waits() {
+    if (!abandoned()) return;
+    told = true;
+    throw std::runtime_error("Gauss-Seidel sweep: a wait between tiles ran out (the sweep was abandoned)");
   }
   // optional per-phase CUDA-event timing on the engine stream
   bool profiling = false;
@@ -2299,10 +2302,42 @@ Engine::~Engine() {
   }
 }
 
+namespace {
+double *field_ptr(DeviceState &D, const Meta &M, int f, long *n);
+}
+
+// The state at creation again, after an abandoned sweep that has been reported
+// (the stream is idle): every field, the CG's vectors, the solids' temperatures,
+// no assembled matrix, no wait given up.  The sweeps' predictions and the running counters stay.
+void Engine::restart() {
+  DeviceState &D = *d_;
+  cudaStream_t s = D.stream;
+  for (int f = 0; f <= HS_F_P_PRIME; ++f) {
+    long n;
+    double *p = field_ptr(D, case_.fluid, f, &n);
+    if (p) HS_CUDA(cudaMemsetAsync(p, 0, sizeof(double) * (size_t)n, s));
+  }
+  for (double *p : {D.F.r, D.F.pa, D.F.pb, D.F.s})
+    HS_CUDA(cudaMemsetAsync(p, 0, sizeof(double) * (size_t)case_.fluid.npad(), s));
+  const std::vector<double> tf(case_.fluid.npad(), prm_.t_fluid0), ts((size_t)D.ntt, prm_.t_solid0);
+  HS_CUDA(cudaMemcpyAsync(D.F.tt, tf.data(), tf.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+  if (D.ntt) HS_CUDA(cudaMemcpyAsync(D.stt, ts.data(), ts.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+  HS_CUDA(cudaMemsetAsync(&D.stats->gave_up, 0, sizeof(int), s));
+  HS_CUDA(cudaStreamSynchronize(s));
+  D.have_matrix = false;
+  *(volatile int *)D.gave_up = 0;
+  D.told = false;
+}
+
 void Engine::init() {
   HS_CUDA(cudaSetDevice(device_));
   DeviceState &D = *d_;
   cudaStream_t s = D.stream;
+  HS_CUDA(cudaStreamSynchronize(s));
+  if (D.abandoned()) {
+    if (!D.told) D.check_waits();
+    restart();
+  }
   long nplane = std::max({(D.F.cz + 2) * (D.F.cy + 2), (D.F.cz + 2) * (D.F.cx + 2), (D.F.cy + 2) * (D.F.cx + 2)});
   for (int which = 0; which < 3; ++which) k_bc<<<grid_for(nplane), kBlock, 0, s>>>(D.F, D.P, which);
   long n = (long)D.F.cx * D.F.cy * D.F.cz;
@@ -2565,7 +2600,7 @@ double *Engine::field_device_ptr(int f, long *n) {
   return field_ptr(*d_, case_.fluid, f, n);
 }
 
-void Engine::check_waits() const { d_->check_waits(); }
+void Engine::check_waits() { d_->check_waits(); }
 
 void Engine::get_field(int f, double *host, long n) {
   HS_CUDA(cudaSetDevice(device_));

@@ -27,7 +27,7 @@ class Engine {
   void sync();
   void set_wait_limit(int polls);
   // throws once the stream has been waited for past a sweep that was abandoned
-  void check_waits() const;
+  void check_waits();
   void stats(hs_stats *out);
   void profile(bool on);
   int profile_read(double *ms, int nphase);
@@ -46,6 +46,7 @@ class Engine {
 
  private:
   void build_multigrid();
+  void restart();
   Case case_;
   hs_params prm_;
   int device_;

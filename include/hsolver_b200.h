@@ -108,7 +108,9 @@ int hs_sync(hs_ctx *ctx);
  * the next call that waits for the stream and reads (hs_sync, hs_step with
  * stats, hs_get_field, hs_get_solid, hs_counters, hs_profile_read, hs_cht_*
  * on the context's flow) returns HS_ERR_INTERNAL.  hs_field_device_ptr does
- * not wait: who reads through it calls hs_sync after hs_step and before. */
+ * not wait: who reads through it calls hs_sync after hs_step and before.  It
+ * stays so until hs_init, which, once the error has been returned, starts
+ * again from the state at creation (every field, the solids included). */
 int hs_set_wait_limit(hs_ctx *ctx, int polls);
 /* The context's cudaStream_t (as void*), for callers that order their own
  * work after hs_step. */

@@ -78,3 +78,34 @@ def test_negative_limit_is_refused():
     with pytest.raises(hsolver_b200.HsError) as e:
         s.set_wait_limit(-1)
     assert e.value.code == -1
+
+
+# a frozen pressure matrix (the default) is assembled once: also that of an
+# abandoned first step must not stay
+@pytest.mark.parametrize("good_steps", [0, 2])
+def test_init_starts_again_after_a_report(good_steps):
+    a, b = _solver(), _solver()
+    a.step(good_steps)
+    a.set_wait_limit(0)
+    a.step(2)
+    _fails(a.sync)
+    a.set_wait_limit(1 << 21)
+    a.init()
+    for n in (1, 2):
+        a.step(n)
+        b.step(n)
+        for f in ("u_star", "v_star", "w_star", "p_temp", "t_temp", "up", "vp", "wp", "ux", "uy", "uz", "p", "t", "p_prime"):
+            assert np.array_equal(a.field(f), b.field(f)), (n, f)
+        for w in ("t_temp", "t"):
+            assert np.array_equal(a.solid(0, w), b.solid(0, w)), (n, w)
+    assert a.counters()["steps"] == good_steps + 2 + 3
+
+
+def test_init_does_not_hide_an_abandoned_step():
+    s = _solver()
+    s.set_wait_limit(0)
+    s.step(1)
+    _fails(s.init)
+    s.set_wait_limit(1 << 21)
+    s.init()
+    s.step(1, stats=True)
