@@ -764,37 +764,33 @@ __device__ void mg_fine_and_rhs(const CgVec<M> &V, const mg::Level<M> &L0, doubl
 // the two passes, but another order of the dot products, and on stretched
 // grids, where a solve takes 40-50 iterations, that moves the fields by 1e-7:
 // the FP64 passes stay per cell.)
-template <int W>
-__device__ __forceinline__ void ldv(float (&v)[W], const float *p, bool cg_) {
-  const float4 t = cg_ ? __ldcg(reinterpret_cast<const float4 *>(p)) : *reinterpret_cast<const float4 *>(p);
+using run::W;
+__device__ __forceinline__ void ldv(float (&v)[W], const float *p) {
+  const float4 t = *reinterpret_cast<const float4 *>(p);
   v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
 }
-template <int W>
 __device__ __forceinline__ void stv(float *p, const float (&v)[W]) {
   *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
 // p = z + beta p_old (or z in the first iteration) at the run q0
-template <class M, int W>
-__device__ __forceinline__ void p_run(M (&v)[W], const M *zs, const M *po, int q0, bool first, M bm) {
-  ldv(v, zs + q0, false);
+__device__ __forceinline__ void p_run(float (&v)[W], const float *zs, const float *po, int q0, bool first, float bm) {
+  ldv(v, zs + q0);
   if (!first) {
-    M o[W];
-    ldv(o, po + q0, false);
+    float o[W];
+    ldv(o, po + q0);
 #pragma unroll
     for (int c = 0; c < W; ++c) v[c] = v[c] + bm * o[c];
   }
 }
-template <class M>
-__device__ __forceinline__ M p_one(const M *zs, const M *po, int q, bool first, M bm) {
-  const M z = zs[q];
+__device__ __forceinline__ float p_one(const float *zs, const float *po, int q, bool first, float bm) {
+  const float z = zs[q];
   return first ? z : z + bm * po[q];
 }
 
 // s = A p with the new p formed on the way (k_ch_pcg's first pass); returns
 // this thread's share of <s, p>
-template <class M>
-__device__ double cg_ap_runs(const CgVec<M> &V, const M *zs, const M *po, M *pn, bool first, M bm, int tid, int T) {
-  constexpr int W = run::Run<M>::W;
+__device__ double cg_ap_runs(const CgVec<float> &V, const float *zs, const float *po, float *pn, bool first, float bm,
+                             int tid, int T) {
   const int N0 = V.N0, PX = V.px, PY = V.N1 + 2, PXY = V.px * (V.N1 + 2);
   double acc = 0.0;
   for (mg::Walk w(PX / W, V.N1, V.N2, tid, T); w.ok(); w.next()) {
@@ -802,14 +798,14 @@ __device__ double cg_ap_runs(const CgVec<M> &V, const M *zs, const M *po, M *pn,
     // the sums d = cw + ce + cs + cn + cb + cf and o = cw pW + ce pE + cs pS
     // + cn pN + cb pB + cf pF built up in that order, one neighbour run at a
     // time (fewer values live at once)
-    M pc[W + 2], g[W + 1], v[W], h[W];
+    float pc[W + 2], g[W + 1], v[W], h[W];
     double d[W], o[W];
     p_run(v, zs, po, q0, first, bm);
     pc[0] = p_one(zs, po, q0 - 1, first, bm);
 #pragma unroll
     for (int c = 0; c < W; ++c) pc[c + 1] = v[c];
     pc[W + 1] = p_one(zs, po, q0 + W, first, bm);
-    ldv(v, V.acx + q0, false);
+    ldv(v, V.acx + q0);
 #pragma unroll
     for (int c = 0; c < W; ++c) g[c] = v[c];
     g[W] = V.acx[q0 + W];
@@ -819,31 +815,31 @@ __device__ double cg_ap_runs(const CgVec<M> &V, const M *zs, const M *po, M *pn,
       o[c] = (double)g[c] * (double)pc[c] + (double)g[c + 1] * (double)pc[c + 2];
     }
     p_run(v, zs, po, q0 - PX, first, bm);
-    ldv(h, V.acy + q0, false);
+    ldv(h, V.acy + q0);
 #pragma unroll
     for (int c = 0; c < W; ++c) { d[c] = d[c] + (double)h[c]; o[c] = o[c] + (double)h[c] * (double)v[c]; }
     p_run(v, zs, po, q0 + PX, first, bm);
-    ldv(h, V.acy + q0 + PX, false);
+    ldv(h, V.acy + q0 + PX);
 #pragma unroll
     for (int c = 0; c < W; ++c) { d[c] = d[c] + (double)h[c]; o[c] = o[c] + (double)h[c] * (double)v[c]; }
     p_run(v, zs, po, q0 - PXY, first, bm);
-    ldv(h, V.acz + q0, false);
+    ldv(h, V.acz + q0);
 #pragma unroll
     for (int c = 0; c < W; ++c) { d[c] = d[c] + (double)h[c]; o[c] = o[c] + (double)h[c] * (double)v[c]; }
     p_run(v, zs, po, q0 + PXY, first, bm);
-    ldv(h, V.acz + q0 + PXY, false);
-    M pv[W], sv[W];
+    ldv(h, V.acz + q0 + PXY);
+    float pv[W], sv[W];
 #pragma unroll
     for (int c = 0; c < W; ++c) {
       d[c] = d[c] + (double)h[c];
       o[c] = o[c] + (double)h[c] * (double)v[c];
       const int i = W * w.m + c;  // padded x
       const bool in = i >= 1 && i <= N0;
-      const M p0 = pc[c + 1];
+      const float p0 = pc[c + 1];
       const double s_ = d[c] * (double)p0 - o[c];
-      pv[c] = in ? p0 : M(0);
-      sv[c] = in ? (M)s_ : M(0);
-      if (in) acc += (double)(M)s_ * (double)p0;
+      pv[c] = in ? p0 : 0.0f;
+      sv[c] = in ? (float)s_ : 0.0f;
+      if (in) acc += (double)(float)s_ * (double)p0;
     }
     stv(pn + q0, pv);
     stv(V.s + q0, sv);
@@ -851,39 +847,37 @@ __device__ double cg_ap_runs(const CgVec<M> &V, const M *zs, const M *po, M *pn,
   return acc;
 }
 
-// x += alpha p, r -= alpha s and, with the V-cycle, its level-0 right-hand
-// side r and the seed of the first half-sweep (x = r / d on colour 0; colour
+// x += alpha p, r -= alpha s (the V-cycle's level-0 right-hand side) and, with
+// the V-cycle, the seed of the first half-sweep (x = r / d on colour 0; colour
 // 1, which the next half-sweep writes before any pass reads it, gets 0);
 // returns this thread's share of <r, r>
-template <class M>
-__device__ double cg_update_runs(const CgVec<M> &V, const mg::Level<M> &L0, bool pre, const M *pn, double alpha,
-                                 int tid, int T) {
-  constexpr int W = run::Run<M>::W;
+__device__ double cg_update_runs(const CgVec<float> &V, const mg::Level<float> &L0, bool pre, const float *pn,
+                                 double alpha, int tid, int T) {
   const int N0 = V.N0, PX = V.px, PY = V.N1 + 2;
   double acc = 0.0;
   for (mg::Walk w(PX / W, V.N1, V.N2, tid, T); w.ok(); w.next()) {
     const int q0 = W * w.m + PX * ((w.j + 1) + PY * (w.k + 1));
-    M xv[W], pv[W], rv[W], sv[W], dv[W];
-    ldv(xv, V.x + q0, false);
-    ldv(pv, pn + q0, false);
-    ldv(rv, V.r + q0, false);
-    ldv(sv, V.s + q0, false);
-    if (pre) ldv(dv, L0.d + q0, false);
+    float xv[W], pv[W], rv[W], sv[W], dv[W];
+    ldv(xv, V.x + q0);
+    ldv(pv, pn + q0);
+    ldv(rv, V.r + q0);
+    ldv(sv, V.s + q0);
+    if (pre) ldv(dv, L0.d + q0);
     else
 #pragma unroll
-      for (int c = 0; c < W; ++c) dv[c] = M(0);
-    M xo[W], ro[W], sx[W];
+      for (int c = 0; c < W; ++c) dv[c] = 0.0f;
+    float xo[W], ro[W], sx[W];
 #pragma unroll
     for (int c = 0; c < W; ++c) {
       const int i = W * w.m + c;
       const bool in = i >= 1 && i <= N0;
-      const M xn = (M)((double)xv[c] + alpha * (double)pv[c]);
-      const M rn = (M)((double)rv[c] - alpha * (double)sv[c]);
+      const float xn = (float)((double)xv[c] + alpha * (double)pv[c]);
+      const float rn = (float)((double)rv[c] - alpha * (double)sv[c]);
       xo[c] = in ? xn : xv[c];
       ro[c] = in ? rn : rv[c];
       if (in) acc += (double)rn * (double)rn;
       const bool red = in && !(((i - 1) + w.j + w.k) & 1);
-      sx[c] = red ? (dv[c] == M(0) ? M(0) : rn / dv[c]) : M(0);
+      sx[c] = red ? (dv[c] == 0.0f ? 0.0f : rn / dv[c]) : 0.0f;
     }
     stv(V.x + q0, xo);
     stv(V.r + q0, ro);
@@ -958,7 +952,7 @@ __global__ void __launch_bounds__(PcgT<M>::v, 1)
     };
     // p in storage precision; the product in FP64 (in FP32 its cancellation
     // error for smooth p would reach the near-null modes of the p' system)
-    if constexpr (is_mixed(M())) acc = cg_ap_runs(V, (const M *)(precond ? L0.x : V.r), (const M *)po, pn, first, bm, tid, T);
+    if constexpr (is_mixed(M())) acc = cg_ap_runs(V, precond ? L0.x : V.r, po, pn, first, bm, tid, T);
     else for (mg::Walk w(N0, N1, V.N2, tid, T); w.ok(); w.next()) {
       const int q = (w.m + 1) + PX * ((w.j + 1) + PY * (w.k + 1));
       const M p0 = pval(q);
@@ -974,7 +968,7 @@ __global__ void __launch_bounds__(PcgT<M>::v, 1)
     if (sp == 0.0) break;
     const double alpha = gamma / sp;
     acc = 0.0;
-    if constexpr (is_mixed(M())) acc = cg_update_runs(V, L0, precond != 0, (const M *)pn, alpha, tid, T);
+    if constexpr (is_mixed(M())) acc = cg_update_runs(V, L0, precond != 0, pn, alpha, tid, T);
     else for (mg::Walk w(N0, N1, V.N2, tid, T); w.ok(); w.next()) {
       const int q = (w.m + 1) + PX * ((w.j + 1) + PY * (w.k + 1));
       const bool seed = precond && !((w.m + w.j + w.k) & 1);  // the V-cycle's rhs is r itself

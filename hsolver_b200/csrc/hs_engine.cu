@@ -35,6 +35,7 @@
 #include <string>
 
 #include "hs_engine.hpp"
+#include "hs_mg.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -154,16 +155,7 @@ __device__ double grid_sum(double v, double *partials, int &buf, double *sh, cg:
   if (threadIdx.x == 0) pp[blockIdx.x] = b;
   grid.sync();
   if (threadIdx.x < 32) {
-    // eight loads in flight (one after another: five trips to L2 for 148 blocks)
-    double a = 0.0;
-    for (int q0 = threadIdx.x; q0 < (int)gridDim.x; q0 += 256) {
-      double w[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) w[u] = q0 + 32 * u < (int)gridDim.x ? __ldcg(pp + q0 + 32 * u) : 0.0;
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (q0 + 32 * u < (int)gridDim.x) a += w[u];
-    }
+    double a = mg::lane_sum(pp, (int)gridDim.x, 1);
     for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (threadIdx.x == 0) sh[32] = a;
   }
@@ -1926,7 +1918,7 @@ struct DeviceState {
   DevStats *stats = nullptr;
   DevStats *stats_host = nullptr;
   // solids
-  int nreg = 0, solid_blocks = 0, maxS = 0;
+  int nreg = 0, solid_blocks = 0;
   int nsol_block = 0, nsol_coop = 0, sol_smem = 0;  // regions solved by one block each, by the cooperative kernel
   SolidReg *regs = nullptr, *regs_block = nullptr, *regs_coop = nullptr;
   int *sol_hyp = nullptr;        // k_solid_block: hyperplane offsets, cell lists
@@ -2135,7 +2127,6 @@ Engine::Engine(const Case &c, const hs_params &p, int device) : case_(c), prm_(p
     tt_h.insert(tt_h.end(), S.npad(), p.t_solid0);
     tc_h.insert(tc_h.end(), S.ncell(), 0.0);
     em_h.insert(em_h.end(), c.solid_empty[r].begin(), c.solid_empty[r].end());
-    D.maxS = std::max<int>(D.maxS, (int)(S.cx + S.cy + S.cz - 2));
   }
   D.ntt = (long long)tt_h.size(); D.ntc = (long long)tc_h.size();
   D.stt = D.upload(tt_h); D.stc = D.upload(tc_h); D.sem = D.upload(em_h);

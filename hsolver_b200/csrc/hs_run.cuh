@@ -21,30 +21,26 @@ namespace run {
 
 namespace cg = cooperative_groups;
 
-template <class M>
+using M = float;                 // the value type: the FP64 passes stay per cell
+constexpr int W = 4, H = W / 2;  // cells of a run (16 bytes), its cells of one colour
 struct Run {
-  static constexpr int W = 16 / (int)sizeof(M);
   M v[W];
 };
-__device__ __forceinline__ Run<float> ld(const float *p) {
+__device__ __forceinline__ Run ld(const M *p) {
   const float4 t = *reinterpret_cast<const float4 *>(p);
   return {{t.x, t.y, t.z, t.w}};
 }
-__device__ __forceinline__ void st(float *p, const Run<float> &r) {
+__device__ __forceinline__ void st(M *p, const Run &r) {
   *reinterpret_cast<float4 *>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
 }
 // value 2 b + odd of a run; the one before and after it (l, r: the values beyond the run's ends)
-template <class M>
-__device__ __forceinline__ M sel(const Run<M> &x, int b, int odd) {
+__device__ __forceinline__ M sel(const Run &x, int b, int odd) {
   return odd ? x.v[2 * b + 1] : x.v[2 * b];
 }
-template <class M>
-__device__ __forceinline__ M before(const Run<M> &x, int b, int odd, M l) {
+__device__ __forceinline__ M before(const Run &x, int b, int odd, M l) {
   return odd ? x.v[2 * b] : (b > 0 ? x.v[b > 0 ? 2 * b - 1 : 0] : l);
 }
-template <class M>
-__device__ __forceinline__ M after(const Run<M> &x, int b, int odd, M r) {
-  constexpr int W = Run<M>::W;
+__device__ __forceinline__ M after(const Run &x, int b, int odd, M r) {
   return odd ? (2 * b + 2 < W ? x.v[2 * b + 2 < W ? 2 * b + 2 : 0] : r) : x.v[2 * b + 1];
 }
 
@@ -56,10 +52,9 @@ enum { kSmooth = 0, kProlong = 1 };
 
 // One half-sweep of colour c of level F (KIND kProlong: with the prolongation
 // from C fused, as mg::prolong_smooth), in units of 32 runs x zc planes
-template <int KIND, class M>
+template <int KIND>
 __device__ __forceinline__ void sweep(const mg::Level<M> &F, const mg::Level<M> &C, int c, int zc,
                                       const Warps &wk) {
-  constexpr int W = Run<M>::W, H = W / 2;
   const int PX = F.px, PXY = F.px * (F.ny + 2), RP = F.px / W, np = RP * F.ny;
   const int nwc = (np + 31) / 32, units = nwc * ((F.nz + zc - 1) / zc);
   const int CPX = C.px, CPXY = C.px * (C.ny + 2);
@@ -69,15 +64,15 @@ __device__ __forceinline__ void sweep(const mg::Level<M> &F, const mg::Level<M> 
     const int j = e / RP, m = e - j * RP, i0 = W * m - 1;  // i0: the run's first cell
     const int k0 = z * zc, k1 = min(F.nz, k0 + zc);
     int q = W * m + PX * ((j + 1) + (F.ny + 2) * (k0 + 1));
-    Run<M> xm = ld(F.x + q - PXY), xc = ld(F.x + q), bl = ld(F.gz + q);
+    Run xm = ld(F.x + q - PXY), xc = ld(F.x + q), bl = ld(F.gz + q);
     for (int k = k0; k < k1; ++k, q += PXY) {
-      const Run<M> xp = ld(F.x + q + PXY), xs = ld(F.x + q - PX), xn = ld(F.x + q + PX);
+      const Run xp = ld(F.x + q + PXY), xs = ld(F.x + q - PX), xn = ld(F.x + q + PX);
       const M xl = F.x[q - 1], xr = F.x[q + W];
-      const Run<M> gx = ld(F.gx + q), gs = ld(F.gy + q), gn = ld(F.gy + q + PX), bh = ld(F.gz + q + PXY),
-                   rh = ld(F.rhs + q);
+      const Run gx = ld(F.gx + q), gs = ld(F.gy + q), gn = ld(F.gy + q + PX), bh = ld(F.gz + q + PXY),
+                rh = ld(F.rhs + q);
       const M gr = F.gx[q + W];
       const int pa = (i0 + j + k + c) & 1;  // the run's first cell of colour c
-      Run<M> o = xc;
+      Run o = xc;
 #pragma unroll
       for (int b = 0; b < H; ++b) {
         const int i = i0 + 2 * b + pa;
@@ -120,17 +115,15 @@ __device__ __forceinline__ void sweep(const mg::Level<M> &F, const mg::Level<M> 
 
 // The residuals of a run's colour-0 cells in row j, plane k, one per pair of
 // values; 0 outside the level
-template <class M>
-__device__ __forceinline__ void residuals(const mg::Level<M> &F, int m, int j, int k, M (&res)[Run<M>::W / 2]) {
-  constexpr int W = Run<M>::W, H = W / 2;
+__device__ __forceinline__ void residuals(const mg::Level<M> &F, int m, int j, int k, M (&res)[H]) {
   const int PX = F.px, PXY = F.px * (F.ny + 2);
   const bool ok = j < F.ny && k < F.nz;
   const int q = ok ? W * m + PX * ((j + 1) + (F.ny + 2) * (k + 1)) : PXY + PX;
-  const Run<M> xc = ld(F.x + q), xs = ld(F.x + q - PX), xn = ld(F.x + q + PX), xm = ld(F.x + q - PXY),
-               xp = ld(F.x + q + PXY);
+  const Run xc = ld(F.x + q), xs = ld(F.x + q - PX), xn = ld(F.x + q + PX), xm = ld(F.x + q - PXY),
+            xp = ld(F.x + q + PXY);
   const M xl = F.x[q - 1], xr = F.x[q + W];
-  const Run<M> gx = ld(F.gx + q), gs = ld(F.gy + q), gn = ld(F.gy + q + PX), bl = ld(F.gz + q), bh = ld(F.gz + q + PXY),
-               rh = ld(F.rhs + q);
+  const Run gx = ld(F.gx + q), gs = ld(F.gy + q), gn = ld(F.gy + q + PX), bl = ld(F.gz + q), bh = ld(F.gz + q + PXY),
+            rh = ld(F.rhs + q);
   const M gr = F.gx[q + W];
   const int i0 = W * m - 1, pa = (i0 + j + k) & 1;
 #pragma unroll
@@ -153,9 +146,7 @@ __device__ __forceinline__ void residuals(const mg::Level<M> &F, int m, int j, i
 // children's residuals in (dk, dj) order, and the coarse seed).  A lane takes
 // one fine run of a coarse row; its coarse cells begin at the odd values of
 // the run, so the last one's second children are the next lane's.
-template <class M>
 __device__ __forceinline__ void restrict_level(const mg::Level<M> &F, const mg::Level<M> &C, const Warps &wk) {
-  constexpr int W = Run<M>::W, H = W / 2;
   const int RP = F.px / W, np = RP * C.ny, nwc = (np + 30) / 31, units = nwc * C.nz;
   const int lane = threadIdx.x & 31;
   for (int u = wk.id; u < units; u += wk.n) {
@@ -192,9 +183,8 @@ __device__ __forceinline__ void restrict_level(const mg::Level<M> &F, const mg::
 // rounds of (planes + 1 to start a march), at most 6 (longer marches spread
 // the warps over more of the level at a time: 203x75x110 2.41 ms per p' solve
 // with up to 16, 2.31 with up to 6, 2.42 with up to 4, 2.50 with up to 2)
-template <class M>
 inline int pick_planes(const mg::Level<M> &L, int nw) {
-  const long long nwc = ((long long)L.px / Run<M>::W * L.ny + 31) / 32;
+  const long long nwc = ((long long)L.px / W * L.ny + 31) / 32;
   int best = 1;
   long long cost = -1;
   for (int z = 1; z <= 6; ++z) {
@@ -206,7 +196,7 @@ inline int pick_planes(const mg::Level<M> &L, int nw) {
 
 // The V-cycle of mg::vcycle with levels 0..G.nrun - 1 (none of them handled by
 // block 0 alone) in run passes
-template <bool RO, class M>
+template <bool RO>
 __device__ __forceinline__ void vcycle(const mg::Hier<M> &G, cg::grid_group &grid, int tid, int T) {
   const int nwb = blockDim.x >> 5;
   const Warps wk{(int)(blockIdx.x * nwb + (threadIdx.x >> 5)), (int)gridDim.x * nwb};
