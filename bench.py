@@ -75,8 +75,8 @@ MG_SWEEPS = 2
 # p' solve, correction, energy assembly, energy BiCGStab, energy relaxation
 LAUNCHES_PER_STEP = 11
 # DRAM bytes per CG iteration of k_ch_pcg on this case, from one ncu capture
-# (profiles/k_ch_pcg_config2.md: 18.30 GB per 8-iteration launch)
-PCG_TRAFFIC_PER_ITER = 18.30e9 / 8
+# of three 8-iteration launches (17.69 GB each)
+PCG_TRAFFIC_PER_ITER = 17.69e9 / 8
 
 
 def workload(name=NAME, seed=0, host_side=False):

@@ -759,11 +759,10 @@ __device__ void mg_fine_and_rhs(const CgVec<M> &V, const mg::Level<M> &L0, doubl
 // cells and the row's padding) compute from in-bounds loads and store the
 // zeros those cells hold.  Every interior cell's arithmetic is the per-cell
 // pass's, term for term; only the order of this thread's dot-product terms
-// differs.  Mixed p' solve per outer step at 256x128x128: 3.39 ms per cell,
-// 3.11 ms by runs.  (FP64 by runs of two: 95 against 132 us per iteration for
-// the two passes, but another order of the dot products, and on stretched
-// grids, where a solve takes 40-50 iterations, that moves the fields by 1e-7:
-// the FP64 passes stay per cell.)
+// differs.  The two passes at 256x128x128: 94 us per iteration per cell, 58 by
+// runs.  (FP64 by runs of two: 95 against 132 us, but another order of the dot
+// products, and on stretched grids, where a solve takes 40-50 iterations, that
+// moved the fields by up to 8e-7: the FP64 passes stay per cell.)
 using run::W;
 __device__ __forceinline__ void ldv(float (&v)[W], const float *p) {
   const float4 t = *reinterpret_cast<const float4 *>(p);
@@ -1400,8 +1399,11 @@ void setup_cg(ChannelState &S, CgVec<R> &V, const uint8_t *solid, size_t np) {
 
 // The smallest level in run passes (hs_run.cuh).  A smaller one's pass is a
 // grid barrier and a round trip of loads, which the per-cell passes spread
-// over more threads: 128x64x64 alone takes 3.9 us per half-sweep per cell and
-// 4.0-4.2 by runs; 203x75x110 (1.7 million cells) gains (hs_run.cuh).
+// over more threads.  Level 0 per cell -> by runs, ms per p' solve: 96x64x64
+// (0.39 million cells) 1.166 -> 1.212, 128x64x64 (0.52) 1.097 -> 1.123,
+// 131x75x77 (0.76) 1.618 -> 1.598, 160x72x72 (0.83) 1.313 -> 1.286, 128x90x90
+// (1.04) 1.851 -> 1.760, 140x100x100 (1.40) 2.223 -> 2.049: the line lies a
+// little above the crossing.
 constexpr long long kRunCells = 1000000;
 
 template <class M>
@@ -1476,10 +1478,10 @@ CUtensorMap padded_map(EncodeTiled enc, const M *base, int px, int py, int pz, i
   return m;
 }
 
-// The z-marching form of the p' solve when the case allows it: the V-cycle
-// preconditioner on, a coarser level below the finest and level 0 handled
-// grid-wide (not by block 0 alone), p_level0 = 0, and one block of
-// zm::kThreads resident per SM with the ring in shared memory.
+// The z-marching form of the p' solve when it is asked for (p_level0 = 2) and
+// the case allows it: the V-cycle preconditioner on, a coarser level below the
+// finest and level 0 handled grid-wide (not by block 0 alone), and one block
+// of zm::kThreads resident per SM with the ring in shared memory.
 template <class M>
 void setup_zm(ChannelState &S, CgVec<M> &V, mg::Hier<M> &G, PcgMaps &TM, int nsm) {
   S.use_zm = false;
@@ -1928,8 +1930,8 @@ void ch_adjoint(ChannelState *S, double tol, int maxiter, double *J, double *dJd
   CH_CUDA(cudaEventRecord(e0, S->stream));
   cht_forward(S->cht, nullptr, J, fwd_iters, &rel);
   CH_CUDA(cudaEventRecord(e1, S->stream));
-  // the adjoint's time ends with the gradients on the device: their copies
-  // to the host are left out, as the forward's T stays on the device
+  // the adjoint's time ends with the per-cell gradients on the device: the
+  // regions' sums and the copies to the host are left out
   cht_adjoint(S->cht, dJdq, dJdk, adj_iters, &rel, e2);
   CH_CUDA(cudaEventSynchronize(e2));
   float a = 0, b = 0;

@@ -372,7 +372,10 @@ __global__ void k_cht_grad(ChtDev H, const double *T, const double *lam, double 
 }
 
 // dJ/dk per region: block r sums its cells' shares (list: the regions' cells, in
-// cell order from first[r] on) in a fixed order
+// cell order from first[r] on) in a fixed order.  Bound by the round trips of
+// one block's loads: 26-28 us for four to eight regions of at most 24^3 cells,
+// 8.6 ms for one region of 2.6 million at 200x128x128 (the adjoint call there
+// 65 ms with a host loop over copied shares, 57 with this sum)
 __global__ void k_cht_dk(const int *first, const int *list, const double *dk_cell, double *dk) {
   __shared__ double sh[32];
   double a = 0.0;

@@ -355,7 +355,13 @@ constexpr int kGsT = 128;        // threads per block: four warps, spread over t
 // flag, edge loads and release store (~4 us) on top of its steps whatever the
 // number of sweeps, the hyperplane form's barrier serves every sweep in
 // flight (256x128x128 energy: one sweep 0.5 against 1.6 ms, 100 sweeps 34
-// against 15).
+// against 15).  The two cross near four sweeps (ms per solve of u / v / w / T,
+// hyperplanes -> tiles): 24x12x12, 2 sweeps 0.150 / 0.161 / 0.140 / 0.148 ->
+// 0.100 / 0.110 / 0.113 / 0.085, 4 sweeps 0.151 / 0.163 / 0.140 / 0.148 ->
+// 0.151 / 0.167 / 0.171 / 0.128; 50x50x50, 2 sweeps 0.540 / 0.568 / 0.520 /
+// 0.465 -> 0.328 / 0.363 / 0.373 / 0.280, 4 sweeps 0.476 / 0.518 / 0.453 /
+// 0.441 -> 0.423 / 0.467 / 0.479 / 0.357; 256x128x128, 4 sweeps 2.06 / 2.21 /
+// 2.02 / 1.95 -> 2.04 / 2.11 / 2.12 / 1.87.
 constexpr int kTileW = 4;
 constexpr int kGsSpin = 1 << 21; // polls before a wait gives up (about a second), unless set (hs_set_wait_limit)
 constexpr int kGsRing = 32, kGsPitch = 35;  // i values per staged row; its pitch (the lanes' rows and skew in distinct banks)
@@ -1273,8 +1279,11 @@ static_assert(kTX * kTB == 256 && 2 * (kTX + kTY) <= 256, "a group's threads");
 // arrivals, of two groups of 256 threads (126 registers), each with tiles and
 // a named barrier of its own, and the loads of a plane issued a plane ahead.
 // Per iteration, against 256-thread blocks at the registers' occupancy
-// without loads ahead: 50x50x50 12.9 -> 9.9 us, 128^3 50.7 -> 41.4, 256x128x128
-// 97.5 -> 81.7 (one group 116, three or four spill).
+// without loads ahead: in the outer step (k_pcorr) 50x50x50 15.3 -> 9.2 us,
+// 128x64x64 18.7 -> 15.1, 256x128x128 83.6 -> 82.5 (DRAM either way); the
+// stand-alone solve (k_pcg) 128^3 51.9 -> 41.2, 257x131x99 89 -> 72, 256^3
+// 357 -> 302 (one group instead of two: 116 against 82 at 256x128x128; three
+// or four spill).
 constexpr int kCgG = 2, kCgT = 256 * kCgG;
 constexpr int kCgSmem = kCgG * 4 * (kTY + 2) * (kTX + 2) * 8;
 

@@ -7,9 +7,9 @@
 // rate 15.4 us).  Here a thread owns a column of 16-byte runs and marches a
 // few planes in z: the z neighbours stay in registers, every load and store
 // of an array is 16 bytes, and the two x neighbours past the run's ends are
-// scalar loads that hit L1: 13.2 us, and p' solve 3.28 -> 3.01 ms per outer
-// step at 256x128x128, 24.1 -> 20.5 at 512x256x256, 2.42 -> 2.31 at
-// 203x75x110.  An FP64 half-sweep is bound by DRAM either way (201 MB at
+// scalar loads that hit L1: 13.2 us.  p' solve per outer step, per-cell passes
+// -> runs in one build: 256x128x128 3.16 -> 2.90 ms, 512x256x256 21.1 -> 17.3,
+// 203x75x110 2.30 -> 2.22, 131x200x180 14.8 -> 14.3.  An FP64 half-sweep is bound by DRAM either way (201 MB at
 // 256x128x128: 40 us per cell, 42 us by runs of two), so FP64 keeps the
 // per-cell passes.  Every point update is the per-cell pass's expression term
 // for term, so a level's x is theirs bit for bit.
@@ -180,9 +180,11 @@ __device__ __forceinline__ void restrict_level(const mg::Level<M> &F, const mg::
 }
 
 // Planes a thread marches per unit on level L with nw warps: the fewest
-// rounds of (planes + 1 to start a march), at most 6 (longer marches spread
-// the warps over more of the level at a time: 203x75x110 2.41 ms per p' solve
-// with up to 16, 2.31 with up to 6, 2.42 with up to 4, 2.50 with up to 2)
+// rounds of (planes + 1 to start a march), at most 6.  Longer marches spread
+// the warps over more of the level at a time; what that costs or gains is
+// small (ms per p' solve with up to 4 / 6 / 16 planes): 203x75x110 2.31 / 2.22
+// / 2.22, 256x128x128 2.88 / 2.90 / 2.84, 131x200x180 14.6 / 14.3 / 13.9,
+// 512x256x256 17.5 / 17.3 / 17.2
 inline int pick_planes(const mg::Level<M> &L, int nw) {
   const long long nwc = ((long long)L.px / W * L.ny + 31) / 32;
   int best = 1;

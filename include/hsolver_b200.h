@@ -288,7 +288,8 @@ typedef struct hs_channel_params {
                           grid-wide passes), 1 grid-wide passes (one per
                           colour), 2 z-marching passes with TMA-staged planes
                           (both colours of a red-black sweep in one pass)
-                          wherever the grid has a coarser level below it */
+                          wherever the grid has a coarser level below it and
+                          is too large for one block to handle alone */
   int conv;            /* momentum convection, HS_CONV_*: the reference's
                           first-order upwind (fluid_solver.h:441-447, 526-532,
                           609-615), hybrid, or QUICK by deferred correction */
